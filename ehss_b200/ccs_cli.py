@@ -381,11 +381,14 @@ def _trace_group(group, args, modes):
     else:
         torch.cuda.synchronize()
     setup_s = e_build.elapsed_time(e_built) * 1e-3 / len(group)
-    for f, spheres in enumerate(group):
+    if modes.adaptive_pa:
+        from .adaptive_pa import adaptive_pa_runs
+        areas = iter(adaptive_pa_runs([(scenes.scenes[f], row['seed']) for f in range(len(group)) for row in rows[f]],
+                                      args.directions, args.grid_size))
+    for f in range(len(group)):
         for k, row in enumerate(rows[f]):
             if modes.adaptive_pa:
-                from .adaptive_pa import adaptive_pa
-                row['pa'] = adaptive_pa(spheres, args.directions, args.grid_size, row['seed'], scene=scenes.scenes[f])
+                row['pa'] = next(areas)
             if kinds:
                 row['impact_source_s'] = 0.0
             if modes.bvh_pa:
