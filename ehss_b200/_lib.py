@@ -86,6 +86,8 @@ _SIGNATURES = {
     'ehss_source_rays': (ct.c_int, [P, ct.c_int, U64, I64, I64, P, P, P]),
     'ehss_compact_source_rays': (ct.c_int, [P, ct.c_int, U64, I64, I64, P, P, P, P]),
     'ehss_trace': (ct.c_int, [P, I64, ct.c_int, ct.c_int, P, P, P, P, P, P, P, P, P]),
+    'ehss_trace_host_workspace_bytes': (ct.c_int, [I64, P]),
+    'ehss_trace_host': (ct.c_int, [P, I64, ct.c_int, ct.c_int] + [P] * 12 + [U64, P]),
     'ehss_pa_anyhit': (ct.c_int, [P, I64, P, P, P, P, P, P]),
     'ehss_pa_grid_workspace_bytes': (ct.c_int, [I64, ct.c_int, ct.c_int, P]),
     'ehss_pa_grid': (ct.c_int, [P, I64, ct.c_int, U64, ct.c_int, P, P, P, P, U64, P]),

@@ -262,8 +262,103 @@ int ehss_trace(const void* scene_dev, int64_t n_rays, int cap, int precision, do
         set_error("null pointer");
         return EHSS_ERR_VALUE;
     }
-    return launch_trace_rays(scene_dev, n_rays, cap, precision, positions_dev, directions_dev, last_atom_dev,
-                             bounces_dev, escaped_dev, unresolved_dev, history_dev, stats_dev, as_stream(stream));
+    RayBuffers B = {};
+    B.scene = scene_dev; B.n = n_rays; B.cap = cap;
+    B.origins = B.positions = positions_dev;
+    B.directions = B.outgoing = directions_dev;
+    B.last = last_atom_dev;
+    B.bounces = B.bounces_out = bounces_dev;
+    B.escaped = escaped_dev; B.unresolved = unresolved_dev;
+    B.history = history_dev; B.stats = stats_dev;
+    return launch_trace_rays(B, precision, as_stream(stream));
+}
+
+// Workspace of ehss_trace_host: the ray counter and counters of finished runs (zeroed together), then device copies
+// of the results.
+struct HostTraceLayout {
+    uint64_t stats, finished, zeroed, positions, outgoing, bounces, escaped, unresolved, total;
+};
+
+static HostTraceLayout host_trace_layout(int64_t n) {
+    HostTraceLayout L;
+    uint64_t o = 64;                                      // the ray counter
+    L.stats = o; o += 8ull * EHSS_NSTATS;
+    L.finished = o; o += 4ull * ((uint64_t)(n + kExportRays - 1) / kExportRays);
+    L.zeroed = o; o = align256(o);
+    L.positions = o; o = align256(o + 24ull * n);
+    L.outgoing = o; o = align256(o + 24ull * n);
+    L.bounces = o; o = align256(o + 8ull * n);
+    L.escaped = o; o = align256(o + 1ull * n);
+    L.unresolved = o; o = align256(o + 1ull * n);
+    L.total = o + 256;
+    return L;
+}
+
+// Address under which kernels reach p: device memory, or page-locked host memory; 0 for anything else.
+static const void* reachable(const void* p) {
+    cudaPointerAttributes a;
+    if (!p || cudaPointerGetAttributes(&a, p) != cudaSuccess) { cudaGetLastError(); return nullptr; }
+    return a.type == cudaMemoryTypeUnregistered ? nullptr : a.devicePointer;
+}
+
+int ehss_trace_host_workspace_bytes(int64_t n_rays, uint64_t* workspace_bytes) {
+    clear_error();
+    if (!workspace_bytes || n_rays < 0) { set_error("invalid arguments"); return EHSS_ERR_VALUE; }
+    *workspace_bytes = host_trace_layout(n_rays).total;
+    return EHSS_OK;
+}
+
+int ehss_trace_host(const void* scene_dev, int64_t n_rays, int cap, int precision, const double* origins,
+                    const double* directions, const int64_t* last_atom, const int64_t* initial_bounces,
+                    double* positions_host, double* outgoing_host, int64_t* bounces_host, uint8_t* escaped_host,
+                    uint8_t* unresolved_host, int32_t* history_dev, uint64_t* stats_host, void* workspace_dev,
+                    uint64_t workspace_bytes, void* stream) {
+    clear_error();
+    if (cap < 1) { set_error("Positive cap and zero/one initial collision required"); return EHSS_ERR_VALUE; }
+    if (precision != EHSS_PREC_FP64 && precision != EHSS_PREC_FP32) { set_error("unknown precision %d", precision); return EHSS_ERR_VALUE; }
+    if (n_rays < 0) { set_error("negative ray count"); return EHSS_ERR_VALUE; }
+    const HostTraceLayout W = host_trace_layout(n_rays);
+    if (workspace_bytes < W.total) {
+        set_error("trace workspace holds %llu bytes, %llu required", (unsigned long long)workspace_bytes,
+                  (unsigned long long)W.total);
+        return EHSS_ERR_CAPACITY;
+    }
+    RayBuffers B = {};
+    if (n_rays > 0) {
+        B.origins = (const double*)reachable(origins);
+        B.directions = (const double*)reachable(directions);
+        B.last = (const int64_t*)reachable(last_atom);
+        B.bounces = (const int64_t*)reachable(initial_bounces);
+        B.host_positions = (double*)reachable(positions_host);
+        B.host_outgoing = (double*)reachable(outgoing_host);
+        B.host_bounces = (int64_t*)reachable(bounces_host);
+        B.host_escaped = (uint8_t*)reachable(escaped_host);
+        B.host_unresolved = (uint8_t*)reachable(unresolved_host);
+        if (!scene_dev || !workspace_dev || !B.origins || !B.directions || (last_atom && !B.last) ||
+            (initial_bounces && !B.bounces) || !B.host_positions || !B.host_outgoing || !B.host_bounces ||
+            !B.host_escaped || !B.host_unresolved) {
+            set_error("rays and results must lie in device or page-locked host memory");
+            return EHSS_ERR_VALUE;
+        }
+    }
+    if (!stats_host || !workspace_dev) { set_error("null pointer"); return EHSS_ERR_VALUE; }
+    char* const base = (char*)(((uintptr_t)workspace_dev + 255u) & ~(uintptr_t)255u);
+    int rc = cuda_status(cudaMemsetAsync(base, 0, W.zeroed, as_stream(stream)), "trace counters");
+    if (rc) return rc;
+    B.scene = scene_dev; B.n = n_rays; B.cap = cap;
+    B.next = (unsigned long long*)base;
+    B.stats = (uint64_t*)(base + W.stats);
+    B.finished = (unsigned*)(base + W.finished);
+    B.positions = (double*)(base + W.positions);
+    B.outgoing = (double*)(base + W.outgoing);
+    B.bounces_out = (int64_t*)(base + W.bounces);
+    B.escaped = (uint8_t*)(base + W.escaped);
+    B.unresolved = (uint8_t*)(base + W.unresolved);
+    B.history = history_dev;
+    rc = launch_trace_rays(B, precision, as_stream(stream));
+    if (rc) return rc;
+    return cuda_status(cudaMemcpyAsync(stats_host, B.stats, 8ull * EHSS_NSTATS, cudaMemcpyDeviceToHost, as_stream(stream)),
+                       "trace counters");
 }
 
 int ehss_pa_anyhit(const void* scene_dev, int64_t n_rays, const double* origins_dev, const double* directions_dev,

@@ -237,9 +237,27 @@ int build_scenes(int S, const double* const* xyz, const double* const* radii, co
                  cudaStream_t stream, bool exterior = false);
 int refit_scenes(int S, const double* const* xyz, const double* const* radii, const int64_t* n, void* const* scenes,
                  void* workspace, uint64_t workspace_bytes, cudaStream_t stream);
-int launch_trace_rays(const void* scene, int64_t n, int cap, int precision, double* P, double* D,
-                      const int64_t* last, int64_t* bounces, uint8_t* esc, uint8_t* unres, int32_t* hist,
-                      uint64_t* stats, cudaStream_t stream);
+// Rays whose results are copied to the host together (k_rays).
+constexpr int kExportRays = 32;
+// Arrays of one explicit-ray call (k_rays); see ehss_trace and ehss_trace_host.
+struct RayBuffers {
+    const void* scene;
+    int64_t n;
+    int cap;
+    const double *origins, *directions;
+    const int64_t *last, *bounces;
+    double *positions, *outgoing;
+    int64_t* bounces_out;
+    uint8_t *escaped, *unresolved;
+    int32_t* history;
+    uint64_t* stats;
+    unsigned long long* next;
+    unsigned* finished;
+    double *host_positions, *host_outgoing;
+    int64_t* host_bounces;
+    uint8_t *host_escaped, *host_unresolved;
+};
+int launch_trace_rays(const RayBuffers& B, int precision, cudaStream_t stream);
 int launch_pa_rays(const void* scene, int64_t n, const double* P, const double* D, const int64_t* owners,
                    uint8_t* blocked, uint64_t* stats, cudaStream_t stream);
 int launch_sobol_points(int dim, const SobolParams& p, int64_t first, int64_t n, uint32_t* q, cudaStream_t stream);

@@ -397,33 +397,6 @@ __device__ __noinline__ bool anyhit(const SceneView& S, const double* o, const d
     return false;
 }
 
-struct TraceOut {
-    int64_t bounces;
-    bool escaped, unresolved;
-};
-
-// _trace_loop body for one ray (ehss_cpu.py:72-98).  o/d are updated in
-// place; history (may be null) receives input atom ids.
-__device__ __forceinline__ TraceOut trace_ray(const SceneView& S, double* o, double* d, int last_rank,
-                                              int64_t count, int cap, bool exact, int32_t* history,
-                                              LocalStats& st) {
-    TraceOut out;
-    out.escaped = out.unresolved = false;
-    while (true) {
-        double best;
-        int k = exact ? nearest<true>(S, o, d, last_rank, best, st) : nearest<false>(S, o, d, last_rank, best, st);
-        if (k < 0) { out.escaped = true; break; }
-        if (count >= cap) { out.unresolved = true; break; }
-        double4 a = S.atoms64[k];
-        reflect64(o[0], o[1], o[2], d[0], d[1], d[2], a.x, a.y, a.z, a.w, best);
-        if (history) history[count] = S.ids[k];
-        ++count;
-        last_rank = k;
-    }
-    out.bounces = count;
-    return out;
-}
-
 __device__ __forceinline__ void flush_stats(const LocalStats& st, uint64_t* stats) {
     if (!stats) return;
     unsigned v[7] = {st.box, st.sphere, st.queries, st.grazing, st.fallback, st.fp64, st.errors};
@@ -440,56 +413,50 @@ __device__ __forceinline__ void flush_stats(const LocalStats& st, uint64_t* stat
 }
 
 // --------------------------------------------------------------------------
-// Explicit-ray kernels
+// Explicit-ray kernels (EHSS: k_rays, after the Walker it shares with k_blocks)
 // --------------------------------------------------------------------------
-__global__ void __launch_bounds__(128) k_trace_rays(const void* scene, int64_t n, int cap, int exact, double* P,
-                                                    double* D, const int64_t* last_atom, int64_t* bounces,
-                                                    uint8_t* escaped, uint8_t* unresolved, int32_t* history,
-                                                    uint64_t* stats) {
-    SceneView S = scene_view(scene);
-    LocalStats st;
-    int64_t stride = (int64_t)gridDim.x * blockDim.x;
-    int64_t first = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    // exterior scenes hold only the atoms reachable from outside the union: not for arbitrary rays
-    bool ok = S.h->magic == kSceneMagic && S.h->status == 0 && S.h->exterior == 0;
-    for (int64_t i = first; i < n; i += stride) {
-        double o[3] = {P[3 * i], P[3 * i + 1], P[3 * i + 2]};
-        double d[3] = {D[3 * i], D[3 * i + 1], D[3 * i + 2]};
-        int64_t count = bounces[i];
-        int64_t last_id = last_atom[i];
-        int32_t* h = history ? history + i * (int64_t)cap : nullptr;
-        if (!ok || last_id < -1 || last_id >= S.h->n_atoms || count < 0 || count > 1 ||
-            (count == 1 && last_id < 0)) {
-            ++st.errors;
-            escaped[i] = 0; unresolved[i] = 0;
-            continue;
-        }
-        int last_rank = last_id >= 0 ? S.rank[last_id] : -1;
-        if (h && count == 1) h[0] = (int32_t)last_id;
-        TraceOut t = trace_ray(S, o, d, last_rank, count, cap, exact != 0, h, st);
-        P[3 * i] = o[0]; P[3 * i + 1] = o[1]; P[3 * i + 2] = o[2];
-        D[3 * i] = d[0]; D[3 * i + 1] = d[1]; D[3 * i + 2] = d[2];
-        bounces[i] = t.bounces;
-        escaped[i] = t.escaped;
-        unresolved[i] = t.unresolved;
+// Rays [base, base + k) of a caller's [n, 3] array into this lane's a[3] (lane
+// q < k gets ray base + q): the array is read with consecutive lanes on
+// consecutive doubles, so that a page-locked host array crosses PCIe in whole
+// 128-byte reads.  buf: 96 doubles of shared memory of this warp.
+__device__ __forceinline__ void load_rays(const double* src, int64_t base, int k, int q, double* buf, double* a) {
+    const unsigned lane = threadIdx.x & 31;
+    __syncwarp();
+#pragma unroll
+    for (int t = 0; t < 3; ++t) {
+        const int w = lane + 32 * t;
+        if (w < 3 * k) buf[w] = src[3 * base + w];
     }
-    flush_stats(st, stats);
+    __syncwarp();
+    if (q < k) {
+#pragma unroll
+        for (int c = 0; c < 3; ++c) a[c] = buf[3 * q + c];
+    }
 }
 
+// One thread per ray.  origins and directions may lie in page-locked host
+// memory; the kernel then runs at the rate at which they cross PCIe.
 __global__ void __launch_bounds__(128) k_pa_rays(const void* scene, int64_t n, const double* P, const double* D,
                                                  const int64_t* owners, uint8_t* blocked, uint64_t* stats) {
+    __shared__ double buf[4][96];
     SceneView S = scene_view(scene);
     LocalStats st;
-    int64_t stride = (int64_t)gridDim.x * blockDim.x;
+    const unsigned lane = threadIdx.x & 31;
+    const int64_t stride = (int64_t)gridDim.x * blockDim.x;
     // exterior scenes hold only the atoms reachable from outside the union: not for arbitrary rays
     bool ok = S.h->magic == kSceneMagic && S.h->status == 0 && S.h->exterior == 0;
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += stride) {
-        double o[3] = {P[3 * i], P[3 * i + 1], P[3 * i + 2]};
-        double d[3] = {D[3 * i], D[3 * i + 1], D[3 * i + 2]};
+    for (int64_t base = blockIdx.x * (int64_t)blockDim.x + threadIdx.x - lane; base < n; base += stride) {
+        const int k = (int)min((int64_t)32, n - base);
+        double o[3], d[3];
+        load_rays(P, base, k, lane, buf[threadIdx.x >> 5], o);
+        load_rays(D, base, k, lane, buf[threadIdx.x >> 5], d);
+        const int64_t i = base + lane;
+        if (i >= n) continue;
         int64_t owner = owners ? owners[i] : -1;
         if (!ok || owner < -1 || owner >= S.h->n_atoms) { ++st.errors; blocked[i] = 0; continue; }
         blocked[i] = anyhit(S, o, d, owner >= 0 ? S.rank[owner] : -1, st);
     }
+    __syncwarp();
     flush_stats(st, stats);
 }
 
@@ -653,6 +620,29 @@ struct Walker {
         if (h.t[1] != CUDART_INF_F) push(h.ref[1], h.t[1], sdepth);
         return h.ref[0];
     }
+    // One step of a lane: inner nodes until it holds a leaf (the first leaf reached is
+    // held while the lane walks on), then that leaf's tests; the lane's next leaf joins the
+    // next step.  The query is finished when cur == kSentinel and leaf == kNoLeaf.
+    __device__ __forceinline__ void advance(const SceneView& S, int sdepth, int last_rank, const LaneRay& L) {
+        while (cur >= 0 && cur != kSentinel) {
+            const int n_nodes = __ldg(&S.h->n_nodes);
+            if (cur >= n_nodes || ++steps > 2 * n_nodes + 2) { error = true; cur = kSentinel; break; }
+            cur = visit(S.nodes, cur, sdepth);
+            if (cur < 0 && leaf == kNoLeaf) {
+                leaf = cur;
+                cur = pop(sdepth);
+            }
+            if (!__any_sync(__activemask(), leaf == kNoLeaf)) break;
+        }
+        if (leaf != kNoLeaf) {
+            leaf_tests(S, leaf, last_rank, L);
+            leaf = kNoLeaf;
+            if (cur < 0) {
+                leaf = cur;
+                cur = pop(sdepth);
+            }
+        }
+    }
     __device__ __forceinline__ void add_candidate(int k, float lo) {
         if (lo > U) return;
         bool placed = false;
@@ -667,14 +657,10 @@ struct Walker {
         int code = ~ref;
         int first = code >> kLeafBits, cnt = (code & (kMaxLeaf - 1)) + 1;
         if (first + cnt > S.h->n_atoms) { error = true; return; }
+        if (COUNT) sphere += cnt - ((unsigned)(last_rank - first) < (unsigned)cnt ? 1 : 0);
         for (int k = first; k < first + cnt; ++k) {
-            // FILTER: the start atom is excluded after the cheap reject below, which a ray
-            // leaving that atom's surface (moving away from its centre) nearly always takes
-            if (EXACT || COUNT) {
-                if (k == last_rank) continue;
-                if (COUNT) ++sphere;
-            }
             if (EXACT) {
+                if (k == last_rank) continue;
                 double4 a = S.atoms64[k];
                 double t = entry64(L.o[0], L.o[1], L.o[2], L.d[0], L.d[1], L.d[2], a.x, a.y, a.z, a.w);
                 int id = __ldg(S.ids + k);
@@ -690,7 +676,9 @@ struct Walker {
                 float w = fmaf(-vx, vx, fmaf(-vy, vy, fmaf(-vz, vz, a.w * a.w)));
                 float disc = fmaf(b, b, w);
                 if (disc < -r.Edisc || b < -r.Ep) continue;
-                if (!COUNT && k == last_rank) continue;
+                // the start atom is excluded after the cheap reject, which a ray leaving that
+                // atom's surface (moving away from its centre) nearly always takes
+                if (k == last_rank) continue;
                 if (disc >= 2.0f * r.Edisc) {
                     float Et;
                     const float t = b - certain_sqrt(b, disc, r, Et);
@@ -934,7 +922,7 @@ __global__ void __launch_bounds__(128, 8) k_blocks(const ehss_block* blocks, int
             const SceneView S = scene_view(sbase);
             while (true) {
                 if (status == kTraverse) {
-                    // inner nodes; the first leaf reached is held while the lane walks on
+                    // Walker::advance, written out: as a call it costs this kernel 8 bytes of spills and 1 % of its time
                     while (W.cur >= 0 && W.cur != kSentinel) {
                         const int n_nodes = __ldg(&S.h->n_nodes);
                         if (W.cur >= n_nodes || ++W.steps > 2 * n_nodes + 2) { W.error = true; W.cur = kSentinel; break; }
@@ -945,7 +933,6 @@ __global__ void __launch_bounds__(128, 8) k_blocks(const ehss_block* blocks, int
                         }
                         if (!__any_sync(__activemask(), W.leaf == kNoLeaf)) break;
                     }
-                    // one leaf per lane and phase: a lane's next leaf joins the next phase
                     if (W.leaf != kNoLeaf) {
                         W.leaf_tests(S, W.leaf, last_rank, L);
                         W.leaf = kNoLeaf;
@@ -994,6 +981,240 @@ __global__ void __launch_bounds__(128, 8) k_blocks(const ehss_block* blocks, int
 }
 
 // --------------------------------------------------------------------------
+// Explicit rays (EHSS), the Walker and phases of k_blocks with per-ray inputs
+// and outputs.  A lane whose ray has finished takes the next ray of the whole
+// call (a shared counter), so a warp's lanes stay busy until the call's rays
+// are used up; one thread per ray left a warp running until its longest path.
+// Rays are read where they lie: device memory, or page-locked host memory
+// (whole 128-byte PCIe reads, load_rays).  Results go to device arrays; when
+// the caller wants them in page-locked host memory too, the lane whose ray
+// completes a run of kExportRays consecutive rays has its warp copy the run's
+// results there (whole lines again), so reading, tracing and writing back
+// overlap in one launch.  Nothing waits: a run is copied by whoever finishes it.
+// Bound by latency: long-scoreboard stalls (nodes, atoms and, at the ends, the
+// host's memory) take 12 of 20 cycles an instruction.  2000 atoms, 262,144 rays,
+// FP32: 412 us on device arrays (one thread per ray: 620 us) and 660 us with
+// rays and results in host memory (35 copies on two streams around four
+// launches: 1500 us); runs of 32 rays leave sooner than runs of 256 (700 us),
+// and 6 CTAs of 80 registers beat 8 of 64 there (713 us).
+// --------------------------------------------------------------------------
+constexpr int kRayCtas = 6, kRayResolve = 28;     // CTAs per SM; finished lanes that start a resolve phase
+
+struct RayCall {
+    const void* scene;
+    int64_t n;
+    int cap;
+    const double *P, *D;               // source rays; may equal Po, Do
+    const int64_t *last, *bounces;     // NULL: -1 and 0 for every ray
+    double *Po, *Do;                   // results (device)
+    int64_t* bounces_out;
+    uint8_t *escaped, *unresolved;
+    int32_t* history;
+    uint64_t* stats;
+    unsigned long long* next;          // rays handed out; NULL: warps take fixed runs of 32 in turn
+    unsigned* finished;                // per run of kExportRays rays; NULL: results stay on the device
+    double *hP, *hD;                   // page-locked copies of the results
+    int64_t* hb;
+    uint8_t *he, *hu;
+};
+
+struct RayAcc {
+    unsigned queries, grazing, fallback, fp64, errors, pad;
+    double buf[96];
+};
+
+// Copies bytes [begin, end) of a result array to its host copy, 16 bytes a lane where both are aligned.
+__device__ __forceinline__ void export_bytes(void* dst, const void* src, int64_t begin, int64_t end) {
+    const unsigned lane = threadIdx.x & 31;
+    char* d = (char*)dst;
+    const char* s = (const char*)src;
+    if (!(((uintptr_t)(d + begin) | (uintptr_t)(s + begin)) & 15u)) {
+        for (int64_t i = begin + 16 * lane; i + 16 <= end; i += 512) *(uint4*)(d + i) = __ldcg((const uint4*)(s + i));
+        begin += (end - begin) & ~(int64_t)15;
+    }
+    for (int64_t i = begin + lane; i < end; i += 32) d[i] = __ldcg(s + i);
+}
+
+// Counts the warp's finished rays; runs that are complete with them go to the host.
+__device__ __noinline__ void export_runs(const RayCall& C, bool fin, int64_t ray) {
+    bool last_of_run = false;
+    if (fin) {
+        const int64_t g = ray / kExportRays;
+        const unsigned size = (unsigned)min((int64_t)kExportRays, C.n - g * kExportRays);
+        __threadfence();
+        last_of_run = atomicAdd(C.finished + g, 1u) + 1u == size;
+    }
+    for (unsigned todo = __ballot_sync(0xffffffffu, last_of_run); todo; todo &= todo - 1) {
+        const int64_t b = __shfl_sync(0xffffffffu, ray, __ffs(todo) - 1) / kExportRays * kExportRays;
+        const int64_t e = min(b + kExportRays, C.n);
+        __threadfence();
+        export_bytes(C.hP, C.Po, 24 * b, 24 * e);
+        export_bytes(C.hD, C.Do, 24 * b, 24 * e);
+        export_bytes(C.hb, C.bounces_out, 8 * b, 8 * e);
+        export_bytes(C.he, C.escaped, b, e);
+        export_bytes(C.hu, C.unresolved, b, e);
+    }
+}
+
+template <bool EXACT>
+__global__ void __launch_bounds__(128, kRayCtas) k_rays(const __grid_constant__ RayCall C, int resolve_batch, int smem_stack) {
+    const unsigned lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5, full = 0xffffffffu;
+    LaneRay& L = reinterpret_cast<LaneRay*>(smem_raw + sizeof(WarpAcc) * nwarps)[threadIdx.x];
+    RayAcc& A = *reinterpret_cast<RayAcc*>(smem_raw + sizeof(WarpAcc) * nwarps + sizeof(LaneRay) * blockDim.x +
+                                           sizeof(int2) * smem_stack * blockDim.x + sizeof(RayAcc) * warp);
+    const unsigned lt_mask = (1u << lane) - 1u;
+    const SceneHeader* const H = reinterpret_cast<const SceneHeader*>(C.scene);
+    // exterior scenes hold only the atoms reachable from outside the union: not for arbitrary rays
+    const bool ok = H->magic == kSceneMagic && H->status == 0 && H->exterior == 0;
+    if (lane == 0) A.queries = A.grazing = A.fallback = A.fp64 = A.errors = 0;
+    __syncwarp();
+    Walker<EXACT, true> W;
+    W.box = W.sphere = 0;
+    int status = kNeedRay, bounces = 0, last_rank = -1;
+    int64_t ray = 0;
+    // fixed runs (no counter): this warp's current run [pool, pool_end) and its next one
+    int64_t run = 32 * (blockIdx.x * (int64_t)nwarps + warp), pool = run, pool_end = min(run + 32, C.n);
+    bool more = true;
+    while (true) {
+        // ---- resolve finished queries (FP64) ----
+        bool fin = false;
+        if (status == kDone) {
+            const SceneView S = scene_view(C.scene);
+            int k;
+            double best;
+            const bool far = W.steps < 0;             // origin beyond the FP32 bounds: all-atom search
+            if (W.error) {
+                atomicAdd(&A.errors, 1u);
+                k = -1; best = CUDART_INF;
+            } else if (far || (!EXACT && W.overflow)) {
+                if (!EXACT && W.grazing) atomicAdd(&A.grazing, 1u);
+                LocalStats fst;
+                k = nearest<true>(S, L.o, L.d, last_rank, best, fst);
+                if (!far) atomicAdd(&A.fallback, 1u);
+                if (!EXACT) atomicAdd(&A.fp64, fst.fp64);
+                if (fst.errors) atomicAdd(&A.errors, fst.errors);
+                W.box += fst.box;
+                W.sphere += fst.sphere;
+            } else if (EXACT) {
+                k = W.best_rank; best = W.best;
+            } else {
+                if (W.grazing) atomicAdd(&A.grazing, 1u);
+                unsigned f = 0;
+                k = resolve_candidates<true>(S, reinterpret_cast<const Walker<false, true>&>(W), L, best, f);
+                atomicAdd(&A.fp64, f);
+            }
+            if (k < 0 || bounces >= C.cap) {
+#pragma unroll
+                for (int c = 0; c < 3; ++c) { C.Po[3 * ray + c] = L.o[c]; C.Do[3 * ray + c] = L.d[c]; }
+                C.bounces_out[ray] = bounces;
+                C.escaped[ray] = k < 0;
+                C.unresolved[ray] = k >= 0;
+                fin = true;
+                status = kNeedRay;
+            } else {
+                const double4 a = S.atoms64[k];
+                reflect64(L.o[0], L.o[1], L.o[2], L.d[0], L.d[1], L.d[2], a.x, a.y, a.z, a.w, best);
+                if (C.history) C.history[ray * (int64_t)C.cap + bounces] = S.ids[k];
+                ++bounces;
+                last_rank = k;
+                W.reset();
+                if (!setup_ray(S.h, L.o, L.d, W.r, EXACT ? 0.0f : kWidenShortDisc)) { W.steps = -1; W.cur = kSentinel; }
+                atomicAdd(&A.queries, 1u);
+                status = kTraverse;
+            }
+        }
+        if (C.finished && __any_sync(full, fin)) export_runs(C, fin, ray);
+        // ---- new rays for lanes whose ray finished ----
+        bool bad = false;
+        const unsigned need = __ballot_sync(full, status == kNeedRay);
+        const bool refill = need && (__popc(need) >= kNewRayBatch || !more || !__any_sync(full, status == kTraverse));
+        int64_t base = 0;
+        int got = 0;
+        if (refill && more) {
+            const int want = __popc(need);
+            if (C.next) {
+                unsigned long long t = 0;
+                if (lane == 0) t = atomicAdd(C.next, (unsigned long long)want);
+                base = (int64_t)__shfl_sync(full, t, 0);
+                got = (int)max((int64_t)0, min((int64_t)want, C.n - base));
+                more = base + want < C.n;
+            } else {
+                if (pool >= pool_end) {
+                    run += 32 * (int64_t)gridDim.x * nwarps;
+                    pool = run;
+                    pool_end = min(run + 32, C.n);
+                }
+                base = pool;
+                got = (int)max((int64_t)0, min((int64_t)want, pool_end - pool));
+                pool += got;
+                more = got > 0;
+            }
+        }
+        if (refill) {
+            const int q = status == kNeedRay ? __popc(need & lt_mask) : 32;
+            if (got > 0) {
+                double o[3], d[3];
+                load_rays(C.P, base, got, q, A.buf, o);
+                load_rays(C.D, base, got, q, A.buf, d);
+                if (q < got) {
+                    const SceneView S = scene_view(C.scene);
+                    ray = base + q;
+                    const int64_t count = C.bounces ? C.bounces[ray] : 0, last_id = C.last ? C.last[ray] : -1;
+#pragma unroll
+                    for (int c = 0; c < 3; ++c) { L.o[c] = o[c]; L.d[c] = d[c]; }
+                    if (!ok || last_id < -1 || last_id >= S.h->n_atoms || count < 0 || count > 1 || (count == 1 && last_id < 0)) {
+                        atomicAdd(&A.errors, 1u);
+                        if (C.Po != C.P) {
+#pragma unroll
+                            for (int c = 0; c < 3; ++c) { C.Po[3 * ray + c] = o[c]; C.Do[3 * ray + c] = d[c]; }
+                            C.bounces_out[ray] = count;
+                        }
+                        C.escaped[ray] = 0;
+                        C.unresolved[ray] = 0;
+                        bad = true;                       // stays kNeedRay
+                    } else {
+                        if (C.history && count == 1) C.history[ray * (int64_t)C.cap] = (int32_t)last_id;
+                        bounces = (int)count;
+                        last_rank = last_id >= 0 ? S.rank[last_id] : -1;
+                        W.reset();
+                        if (!setup_ray(S.h, L.o, L.d, W.r, EXACT ? 0.0f : kWidenShortDisc)) { W.steps = -1; W.cur = kSentinel; }
+                        atomicAdd(&A.queries, 1u);
+                        status = kTraverse;
+                    }
+                }
+            }
+            if (!more && status == kNeedRay && !(q < got)) status = kIdle;
+        }
+        if (C.finished && __any_sync(full, bad)) export_runs(C, bad, ray);
+        if (!__any_sync(full, status == kTraverse)) {
+            if (!__any_sync(full, status == kNeedRay)) break;
+            continue;
+        }
+        // ---- traverse until enough queries are finished ----
+        const SceneView S = scene_view(C.scene);
+        while (true) {
+            if (status == kTraverse) {
+                W.advance(S, smem_stack, last_rank, L);
+                if (W.cur == kSentinel && W.leaf == kNoLeaf) status = kDone;
+            }
+            // lanes without a ray count towards the batch: the call's last rays do not wait for one another
+            const unsigned trav = __ballot_sync(full, status == kTraverse);
+            if (32 - __popc(trav) >= resolve_batch) break;
+        }
+    }
+    if (!C.stats) return;
+    const unsigned long long box = warp_sum64(W.box), sphere = warp_sum64(W.sphere);
+    __syncwarp();
+    if (lane == 0) {
+        const unsigned long long v[7] = {box, sphere, A.queries, A.grazing, A.fallback, EXACT ? sphere : A.fp64, A.errors};
+        const int slot[7] = {EHSS_STAT_BOX_TESTS, EHSS_STAT_SPHERE_TESTS, EHSS_STAT_QUERIES, EHSS_STAT_GRAZING,
+                             EHSS_STAT_FALLBACK, EHSS_STAT_FP64_TESTS, EHSS_STAT_ERRORS};
+        for (int i = 0; i < 7; ++i)
+            if (v[i]) atomicAdd((unsigned long long*)&C.stats[slot[i]], v[i]);
+    }
+}
+
+// --------------------------------------------------------------------------
 // Host launchers
 // --------------------------------------------------------------------------
 static unsigned grid_for(int64_t n, int threads) {
@@ -1003,12 +1224,25 @@ static unsigned grid_for(int64_t n, int threads) {
     return (unsigned)(want > 0 ? want : 1);
 }
 
-int launch_trace_rays(const void* scene, int64_t n, int cap, int precision, double* P, double* D,
-                      const int64_t* last, int64_t* bounces, uint8_t* esc, uint8_t* unres, int32_t* hist,
-                      uint64_t* stats, cudaStream_t stream) {
-    if (n == 0) return EHSS_OK;
-    k_trace_rays<<<grid_for(n, 128), 128, 0, stream>>>(scene, n, cap, precision == EHSS_PREC_FP64, P, D, last,
-                                                       bounces, esc, unres, hist, stats);
+int launch_trace_rays(const RayBuffers& B, int precision, cudaStream_t stream) {
+    if (B.n == 0) return EHSS_OK;
+    RayCall C;
+    C.scene = B.scene; C.n = B.n; C.cap = B.cap;
+    C.P = B.origins; C.D = B.directions; C.last = B.last; C.bounces = B.bounces;
+    C.Po = B.positions; C.Do = B.outgoing; C.bounces_out = B.bounces_out; C.escaped = B.escaped; C.unresolved = B.unresolved;
+    C.history = B.history; C.stats = B.stats;
+    C.next = B.next; C.finished = B.finished;
+    C.hP = B.host_positions; C.hD = B.host_outgoing; C.hb = B.host_bounces; C.he = B.host_escaped; C.hu = B.host_unresolved;
+    // few rays: one-warp CTAs, so that they spread over the SMs
+    const int64_t warps = (B.n + 31) / 32;
+    const int threads = warps < 4ll * sm_count() ? 32 : 128;
+    const int64_t want = (warps * 32 + threads - 1) / threads, most = (int64_t)sm_count() * kRayCtas;
+    const int sdepth = 5;
+    const size_t smem = sizeof(WarpAcc) * (size_t)(threads / 32) + sizeof(LaneRay) * (size_t)threads +
+                        sizeof(int2) * sdepth * (size_t)threads + sizeof(RayAcc) * (size_t)(threads / 32);
+    const unsigned grid = (unsigned)(want < most ? want : most);
+    if (precision == EHSS_PREC_FP64) k_rays<true><<<grid, threads, smem, stream>>>(C, kRayResolve, sdepth);
+    else k_rays<false><<<grid, threads, smem, stream>>>(C, kRayResolve, sdepth);
     return cuda_status(cudaGetLastError(), "trace launch");
 }
 

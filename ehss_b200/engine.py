@@ -168,17 +168,37 @@ def external_source(spheres, power, seed, scene=None):
                       np.full(n, -1), np.zeros(n, dtype=np.int64), "external impact disk")
 
 
+def _reachable(a, device, hold):
+    """Address of a contiguous host array that kernels can read where it lies
+    (page-locked memory), or of a device copy; ``hold`` keeps it alive."""
+    host = torch().from_numpy(a)
+    t = host if host.is_pinned() else host.to(device)
+    hold.append(t)
+    return t.data_ptr()
+
+
+def _page_locked(device, sizes):
+    """uint8 views of one new page-locked buffer, one per size, each on a 64-byte boundary."""
+    starts, total = [], 0
+    for n in sizes:
+        starts.append(total)
+        total += -(-n // 64) * 64
+    buf = torch().empty(max(total, 1), dtype=torch().uint8, pin_memory=True)
+    return buf, [buf[s:s + n].numpy() for s, n in zip(starts, sizes)]
+
+
+def _ends_equal(a, value):
+    return len(a) > 0 and a[0] == value and a[-1] == value
+
+
 class GPUEHSSTransport:
     """EHSS tracer on one prepared scene (CPUEHSSTransport.trace contract).
 
-    ``trace`` takes and returns host arrays, as the reference does.  The rays
-    go through in up to four chunks on two streams, so one chunk's copy to
-    the device overlaps the previous chunk's trace and copy back; results are
-    copied into page-locked host buffers that become the returned arrays (no
-    second copy).  Device buffers are kept and grown across calls.
+    ``trace`` takes and returns host arrays, as the reference does.  One
+    launch reads the rays from page-locked host memory (rays in pageable
+    arrays are copied to the device first), traces them and writes the results
+    into a page-locked buffer whose parts become the returned arrays.
     """
-
-    PIPELINE_MIN_CHUNK = 1 << 15
 
     def __init__(self, scene, precision='fp32', threads=1):
         if getattr(scene, 'exterior', False):
@@ -186,78 +206,38 @@ class GPUEHSSTransport:
         self.scene = scene
         self.precision = _precision(precision)
         self.threads = threads
-        self._dev = None
-        self._dev_rays = 0
-        self._streams = None
-
-    def _buffers(self, n, cap, record_history):
-        t = torch()
-        dev = self.scene.device
-        if self._dev is None or self._dev_rays < n:
-            self._dev = dict(P=t.empty((n, 3), dtype=t.float64, device=dev), D=t.empty((n, 3), dtype=t.float64, device=dev),
-                             last=t.empty(n, dtype=t.int64, device=dev), bounces=t.empty(n, dtype=t.int64, device=dev),
-                             esc=t.empty(n, dtype=t.uint8, device=dev), unres=t.empty(n, dtype=t.uint8, device=dev))
-            self._dev_rays = n
-        if self._streams is None:
-            self._streams = [t.cuda.Stream(dev), t.cuda.Stream(dev)]
-        hist = t.empty((n, cap), dtype=t.int32, device=dev) if record_history else None
-        return self._dev, hist
 
     def trace(self, source, cap=64, record_history=False):
-        if type(cap) is not int or cap < 1 or cap > np.iinfo(np.int32).max or np.any(source.initial_bounces > 1):
+        if type(cap) is not int or cap < 1 or cap > np.iinfo(np.int32).max:
             raise ValueError('Positive cap and zero/one initial collision required')
-        n_atoms = self.scene.n_atoms
-        if np.any(source.last_atom < -1) or np.any(source.last_atom >= n_atoms):
-            raise ValueError('Invalid initial physical identity')
-        lib = _lib.load()
-        t = torch()
         start = time.perf_counter()
         n = len(source.weights)
-        # host inputs as tensors over the caller's memory (no copy when already contiguous of the right type)
-        host_in = dict(P=t.from_numpy(np.ascontiguousarray(source.origins, dtype=np.float64)),
-                       D=t.from_numpy(np.ascontiguousarray(source.directions, dtype=np.float64)),
-                       last=t.from_numpy(np.ascontiguousarray(source.last_atom, dtype=np.int64)),
-                       bounces=t.from_numpy(np.ascontiguousarray(source.initial_bounces, dtype=np.int64)))
-        d, hist = self._buffers(max(n, 1), cap, record_history)
-        # results land in page-locked buffers that become the returned arrays
-        pin = dict(pin_memory=True)
-        out = dict(P=t.empty((n, 3), dtype=t.float64, **pin), D=t.empty((n, 3), dtype=t.float64, **pin),
-                   bounces=t.empty(n, dtype=t.int64, **pin), esc=t.empty(n, dtype=t.uint8, **pin),
-                   unres=t.empty(n, dtype=t.uint8, **pin))
-        hist_out = t.empty((n, cap), dtype=t.int32, **pin) if record_history else None
-        stats = t.zeros(_lib.NSTATS, dtype=t.int64, device=self.scene.device)
-        main = t.cuda.current_stream(self.scene.device)
-        parts = max(1, min(4, n // self.PIPELINE_MIN_CHUNK))
-        bounds = [n * k // parts for k in range(parts + 1)]
-        for s in self._streams:
-            s.wait_stream(main)           # stats zeroed, buffers free
-        for k in range(parts):
-            a, b = bounds[k], bounds[k + 1]
-            if a == b:
-                continue
-            s = self._streams[k % 2]
-            with t.cuda.stream(s):
-                for key in ('P', 'D', 'last', 'bounces'):
-                    d[key][a:b].copy_(host_in[key][a:b], non_blocking=True)
-                if hist is not None:
-                    hist[a:b].fill_(-1)
-                _lib.check(lib.ehss_trace(self.scene.ptr, b - a, cap, self.precision, ptr(d['P'][a:b]),
-                                          ptr(d['D'][a:b]), ptr(d['last'][a:b]), ptr(d['bounces'][a:b]),
-                                          ptr(d['esc'][a:b]), ptr(d['unres'][a:b]),
-                                          None if hist is None else ptr(hist[a:b]), ptr(stats), s.cuda_stream),
-                           'trace')
-                for key in ('P', 'D', 'bounces', 'esc', 'unres'):
-                    out[key][a:b].copy_(d[key][a:b], non_blocking=True)
-                if hist is not None:
-                    hist_out[a:b].copy_(hist[a:b], non_blocking=True)
-        for s in self._streams:
-            main.wait_stream(s)
-        st = stats.cpu().numpy().astype(np.uint64)       # synchronises the main stream, hence both others
+        origins, directions = (np.ascontiguousarray(a, dtype=np.float64) for a in (source.origins, source.directions))
+        last, bounces = (np.ascontiguousarray(a, dtype=np.int64) for a in (source.last_atom, source.initial_bounces))
+        if origins.shape != (n, 3) or directions.shape != (n, 3) or last.shape != (n,) or bounces.shape != (n,):
+            raise ValueError('One origin, direction, initial identity and bounce count per weight required')
+        # A source starts without colliders (-1) and collisions as a rule.  Where its ends say so, the device traces
+        # it that way while the host reads the two arrays through; if an entry differs, the result is dropped and
+        # the arrays are checked and traced as they are.
+        done = None
+        if _ends_equal(last, -1) and _ends_equal(bounces, 0):
+            done = self._enqueue(origins, directions, None, None, cap, record_history)
+            plain = not bounces.any() and last.max() == -1 and last.min() == -1
+            torch().cuda.current_stream(self.scene.device).synchronize()
+            if not plain:
+                done = None
+        if done is None:
+            if np.any(source.initial_bounces > 1):
+                raise ValueError('Positive cap and zero/one initial collision required')
+            if np.any(last < -1) or np.any(last >= self.scene.n_atoms):
+                raise ValueError('Invalid initial physical identity')
+            done = self._enqueue(origins, directions, last, bounces, cap, record_history)
+            torch().cuda.current_stream(self.scene.device).synchronize()
+        (P, D, b, esc, unres, st), hist_out = done
         if st[_lib.STAT_ERRORS]:
             raise _lib.EHSSDeviceError(f'{int(st[_lib.STAT_ERRORS])} rays reported a bounded device failure')
         history = hist_out.numpy() if record_history else np.full((n, 0), -1, dtype=np.int32)
-        return EHSSResult(out['P'].numpy(), out['D'].numpy(), out['esc'].numpy().view(np.bool_),
-                          out['unres'].numpy().view(np.bool_), out['bounces'].numpy(), history, source,
+        return EHSSResult(P, D, esc, unres, b, history, source,
                           dict(query_s=time.perf_counter() - start, sphere_tests=int(st[_lib.STAT_SPHERE]),
                                box_tests=int(st[_lib.STAT_BOX]), queries=int(st[_lib.STAT_QUERIES]),
                                grazing_queries=int(st[_lib.STAT_GRAZING]),
@@ -266,6 +246,27 @@ class GPUEHSSTransport:
                                precision='fp64' if self.precision == _lib.PREC_FP64 else 'fp32',
                                threads=self.threads, history_recorded=bool(record_history),
                                response_reuse=False))
+
+    def _enqueue(self, origins, directions, last, bounces, cap, record_history):
+        """Enqueue one trace (no wait); returns the host arrays that it fills."""
+        lib, t, dev = _lib.load(), torch(), self.scene.device
+        n = len(origins)
+        hold = []
+        inputs = [None if a is None else _reachable(a, dev, hold) for a in (origins, directions, last, bounces)]
+        wb = ct.c_uint64()
+        _lib.check(lib.ehss_trace_host_workspace_bytes(n, ct.byref(wb)), 'trace')
+        ws = t.empty(wb.value, dtype=t.uint8, device=dev)
+        buf, (P, D, b, esc, unres, st) = _page_locked(dev, (24 * n, 24 * n, 8 * n, n, n, 8 * _lib.NSTATS))
+        hist = t.full((n, cap), -1, dtype=t.int32, device=dev) if record_history else None
+        hist_out = t.empty((n, cap), dtype=t.int32, pin_memory=True) if record_history else None
+        out = [a.ctypes.data for a in (P, D, b, esc, unres)]
+        _lib.check(lib.ehss_trace_host(self.scene.ptr, n, cap, self.precision, *inputs, *out, ptr(hist), st.ctypes.data,
+                                       ws.data_ptr(), wb.value, stream_handle(dev)), 'trace')
+        if hist is not None:
+            hist_out.copy_(hist, non_blocking=True)
+        f8 = np.float64
+        return (P.view(f8).reshape(n, 3), D.view(f8).reshape(n, 3), b.view(np.int64), esc.view(np.bool_),
+                unres.view(np.bool_), st.view(np.uint64)), hist_out
 
 
 def _check_groups(groups, n):
@@ -333,18 +334,36 @@ class SphereIndex:
         owners = getattr(source, 'owners', None)
         if owners is None:
             owners = source.last_atom
-        lib = _lib.load()
-        t = torch()
-        dev = self.scene.device
-        n = len(source.origins)
-        P = to_device(source.origins, np.float64, dev)
-        D = to_device(source.directions, np.float64, dev)
-        own = to_device(owners, np.int64, dev)
-        blocked = t.zeros(n, dtype=t.uint8, device=dev)
-        stats = t.zeros(_lib.NSTATS, dtype=t.int64, device=dev)
-        _lib.check(lib.ehss_pa_anyhit(self.scene.ptr, n, ptr(P), ptr(D), ptr(own), ptr(blocked), ptr(stats),
-                                      stream_handle(dev)), 'PA query')
-        st = stats.cpu().numpy()
+        origins, directions = (np.ascontiguousarray(a, dtype=np.float64) for a in (source.origins, source.directions))
+        own = np.ascontiguousarray(owners, dtype=np.int64)
+        n = len(origins)
+        if origins.shape != (n, 3) or directions.shape != (n, 3) or own.shape != (n,):
+            raise ValueError('One origin, direction and owner per ray required')
+        # rays without an owner (-1) are the rule: traced so while the host reads the owners through (as in trace)
+        done = None
+        if _ends_equal(own, -1):
+            done = self._enqueue(origins, directions, None)
+            plain = own.max() == -1 and own.min() == -1
+            torch().cuda.current_stream(self.scene.device).synchronize()
+            if not plain:
+                done = None
+        if done is None:
+            done = self._enqueue(origins, directions, own)
+            torch().cuda.current_stream(self.scene.device).synchronize()
+        blocked, st = done
         if st[_lib.STAT_ERRORS]:
             raise _lib.EHSSDeviceError('PA query reported a bounded device failure')
-        return blocked.cpu().numpy().astype(bool), int(st[_lib.STAT_BOX]), int(st[_lib.STAT_SPHERE])
+        return blocked, int(st[_lib.STAT_BOX]), int(st[_lib.STAT_SPHERE])
+
+    def _enqueue(self, origins, directions, owners):
+        """Enqueue one any-hit query (no wait); returns the host arrays that it fills."""
+        lib, t, dev = _lib.load(), torch(), self.scene.device
+        n = len(origins)
+        hold = []
+        P, D, own = (None if a is None else _reachable(a, dev, hold) for a in (origins, directions, owners))
+        buf, (blocked, st) = _page_locked(dev, (n, 8 * _lib.NSTATS))
+        stats = t.zeros(_lib.NSTATS, dtype=t.int64, device=dev)
+        _lib.check(lib.ehss_pa_anyhit(self.scene.ptr, n, P, D, own, blocked.ctypes.data if n else None, ptr(stats),
+                                      stream_handle(dev)), 'PA query')
+        t.from_numpy(st.view(np.int64)).copy_(stats, non_blocking=True)
+        return blocked.view(np.bool_), st.view(np.int64)

@@ -218,10 +218,29 @@ int ehss_trace(const void* scene_dev, int64_t n_rays, int cap, int precision,
                int64_t* bounces_dev, uint8_t* escaped_dev, uint8_t* unresolved_dev, int32_t* history_dev,
                uint64_t* stats_dev, void* stream);
 
+/* The same trace for a caller whose rays and results are host arrays
+ * (CPUEHSSTransport.trace takes and returns numpy arrays): one launch reads
+ * the rays where they lie and writes each finished run of results to the
+ * host while others are traced.  origins/directions [n*3], last_atom and
+ * initial_bounces [n] (NULL: -1 and 0 for every ray) and the result arrays
+ * must lie in page-locked host memory (cudaHostAlloc, cudaHostRegister) or
+ * device memory; anything else is EHSS_ERR_VALUE.  The source arrays are not
+ * written.  history_dev as in ehss_trace.  stats_host (page-locked
+ * uint64[EHSS_NSTATS]) receives this call's counters.  Results are complete
+ * when `stream` is.  workspace_dev holds at least
+ * ehss_trace_host_workspace_bytes(n_rays) bytes until then. */
+int ehss_trace_host_workspace_bytes(int64_t n_rays, uint64_t* workspace_bytes);
+int ehss_trace_host(const void* scene_dev, int64_t n_rays, int cap, int precision, const double* origins,
+                    const double* directions, const int64_t* last_atom, const int64_t* initial_bounces,
+                    double* positions_host, double* outgoing_host, int64_t* bounces_host, uint8_t* escaped_host,
+                    uint8_t* unresolved_host, int32_t* history_dev, uint64_t* stats_host, void* workspace_dev,
+                    uint64_t workspace_bytes, void* stream);
+
 /* BVH any-hit PA of explicit rays.  Replaces SphereIndex.query / tree_blocked
  * (pa_spatial.py:133-142, 162-164) with sphere_hit semantics
  * (inside_out_pa.py:93-101): blocked_dev[i] = 1 when ray i meets a sphere
- * other than owners_dev[i] (NULL = no owner). */
+ * other than owners_dev[i] (NULL = no owner).  The arrays may also lie in
+ * page-locked host memory. */
 int ehss_pa_anyhit(const void* scene_dev, int64_t n_rays, const double* origins_dev, const double* directions_dev,
                    const int64_t* owners_dev, uint8_t* blocked_dev, uint64_t* stats_dev, void* stream);
 
