@@ -23,6 +23,7 @@ BLOCK_EHSS, BLOCK_PA = 1, 2
 LAUNCH_COUNT_TESTS = 1
 LAUNCH_RAY_BLOCKS = 2
 LAUNCH_NO_DISK_BLOCKS = 4
+LAUNCH_NO_PA = 8
 # LBVH leaf bound used by default: leaves of 13-16 atoms trace fastest on B200 with the default launch
 DEFAULT_LEAF = 14
 BUILD_EXTERIOR = 1

@@ -91,7 +91,7 @@ class BlockPlan:
         precisions = 0
         for j in jobs:
             precisions |= 1 << int(j.precision)
-        options = _lib.LAUNCH_COUNT_TESTS if L['count_tests'] else 0
+        options = (_lib.LAUNCH_COUNT_TESTS if L['count_tests'] else 0) | (0 if any(j.pa for j in jobs) else _lib.LAUNCH_NO_PA)
         n_boundary = sum(j.boundary is not None for j in jobs)
         if n_boundary:
             options |= _lib.LAUNCH_RAY_BLOCKS | (_lib.LAUNCH_NO_DISK_BLOCKS if n_boundary == len(jobs) else 0)

@@ -482,7 +482,7 @@ static int trace_blocks_impl(const ehss_block* blocks_dev, int n_blocks, int64_t
     }
     if (L.resolve_batch < 1 || L.resolve_batch > 32) { set_error("resolve_batch must be 1..32"); return EHSS_ERR_VALUE; }
     if (L.precisions < 0 || L.precisions > 3) { set_error("precisions must be a mask of 1 and 2 (0 = both)"); return EHSS_ERR_VALUE; }
-    if (L.options & ~(EHSS_LAUNCH_COUNT_TESTS | EHSS_LAUNCH_RAY_BLOCKS | EHSS_LAUNCH_NO_DISK_BLOCKS)) {
+    if (L.options & ~(EHSS_LAUNCH_COUNT_TESTS | EHSS_LAUNCH_RAY_BLOCKS | EHSS_LAUNCH_NO_DISK_BLOCKS | EHSS_LAUNCH_NO_PA)) {
         set_error("unknown launch options 0x%x", L.options);
         return EHSS_ERR_VALUE;
     }

@@ -14,8 +14,9 @@
 // per-thread stack; node boxes are FP32, rounded outward and expanded by eps_box, so a
 // box is culled only when it provably holds no entry at or before the
 // current bound U.  Two sphere-test precisions share the walk:
-//   EXACT (EHSS_PREC_FP64): every reached sphere is tested with the
-//     reference's FP64 formula; U is the running best distance rounded up.
+//   EXACT (EHSS_PREC_FP64): every reached sphere is tested in FP64, with the
+//     reference's formula unless an FP64 discriminant shows a certain miss;
+//     U is the running best distance rounded up.
 //   FILTER (EHSS_PREC_FP32): spheres are tested in FP32 with the
 //     cancellation-free perpendicular-distance discriminant
 //     disc = r^2 - |v - (v.d) d|^2 (the fused kernel: the shorter
@@ -84,6 +85,15 @@ __device__ __forceinline__ bool setup_ray(const SceneHeader* H, const double* o,
     float rm = H->rmax_f;
     r.Edisc = (8.0f * kU32) * rm * rm + 2.5f * rm * r.Ep + 8.0f * r.Ep * r.Ep;
     if (widen > 0.0f) r.Edisc += widen * (rm * rm + A * A);
+    return true;
+}
+
+// setup_ray for the EXACT walk.  Its FP64 reject takes |d| = 1; a direction off by more than 1e-11 in |d|^2 (which
+// moves disc by 1e-11 A^2, below the bounds for A < 10^6 rmax) switches it off with infinite bounds.
+__device__ __forceinline__ bool setup_exact(const SceneHeader* H, const double* o, const double* d, RayF& r) {
+    if (!setup_ray(H, o, d, r)) return false;
+    const double aa = fma(d[0], d[0], fma(d[1], d[1], d[2] * d[2]));
+    if (!(fabs(aa - 1.0) <= 1e-11)) r.Ep = r.Edisc = CUDART_INF_F;
     return true;
 }
 
@@ -658,12 +668,30 @@ struct Walker {
         int first = code >> kLeafBits, cnt = (code & (kMaxLeaf - 1)) + 1;
         if (first + cnt > S.h->n_atoms) { error = true; return; }
         if (COUNT) sphere += cnt - ((unsigned)(last_rank - first) < (unsigned)cnt ? 1 : 0);
+        const double Edisc = EXACT ? (double)r.Edisc : 0., Ep = EXACT ? (double)r.Ep : 0.;
         for (int k = first; k < first + cnt; ++k) {
             if (EXACT) {
+                // FP64 reject before the reference's formula (two divisions and a square root; 650 atoms,
+                // 20 x 65,536 rays with PA: 1.55 -> 1.09 ms together with PA from the first query):
+                // q = x.d, w = |x|^2 - r^2 and disc = q^2 - w are within 1e-13 A^2 of their true
+                // values for unit d (setup_exact), far inside the FP32 filter's bounds
+                const double4 a = S.atoms64[k];
+                const double x0 = L.o[0] - a.x, x1 = L.o[1] - a.y, x2 = L.o[2] - a.z;
+                const double q = fma(x0, L.d[0], fma(x1, L.d[1], x2 * L.d[2]));
+                const double w = fma(x0, x0, fma(x1, x1, fma(x2, x2, -a.w * a.w)));
+                const double disc = fma(q, q, -w);
+                if (disc < -Edisc || q > Ep) continue;                 // certain miss
                 if (k == last_rank) continue;
-                double4 a = S.atoms64[k];
-                double t = entry64(L.o[0], L.o[1], L.o[2], L.d[0], L.d[1], L.d[2], a.x, a.y, a.z, a.w);
-                int id = __ldg(S.ids + k);
+                bool certain = false;
+                if (disc >= 2.0 * Edisc) {
+                    float Et;
+                    const float b = (float)-q, t = b - certain_sqrt(b, (float)disc, r, Et);
+                    if (t < -2.0f * Et || t - Et > U) continue;        // no entry ahead, or behind the best one
+                    certain = t > Et;
+                }
+                if (!certain) grazing = true;
+                const double t = entry64(L.o[0], L.o[1], L.o[2], L.d[0], L.d[1], L.d[2], a.x, a.y, a.z, a.w);
+                const int id = __ldg(S.ids + k);
                 if (better(t, id, best, best_id)) {
                     best = t; best_rank = k; best_id = id;
                     U = __double2float_ru(best);
@@ -754,7 +782,11 @@ __device__ __forceinline__ bool next_chunk(unsigned long long* counters, int n_p
 
 // RAYS: the instance for blocks with EHSS_BLOCK_RAYS (caller-made weighted rays);
 // each instance skips the other kind's chunks, like the precision instances.
-template <bool EXACT, bool COUNT, bool RAYS>
+// PA: the instance that serves EHSS_BLOCK_PA; the caller says with
+// EHSS_LAUNCH_NO_PA that no block has it (such a block is then an error), which
+// keeps the any-hit query's registers out of the kernel (spill stores / loads a
+// thread 112 / 164 -> 88 / 116 B; the 256-globule batch 2 % faster).
+template <bool EXACT, bool COUNT, bool RAYS, bool PA>
 __global__ void __launch_bounds__(128, 8) k_blocks(const ehss_block* blocks, int nb, int64_t chunk_first,
                                                    int64_t total_chunks, int chunk_rays, int resolve_batch,
                                                    ehss_block_result* results,
@@ -790,7 +822,8 @@ __global__ void __launch_bounds__(128, 8) k_blocks(const ehss_block* blocks, int
         // only the scene's base stays live across the phases; each phase rebuilds the view
         // it needs from the (L1-resident) header, which keeps the traversal's registers free
         const void* const sbase = B->scene;
-        const bool ok = scene_view(sbase).h->magic == kSceneMagic && scene_view(sbase).h->status == 0;
+        const bool ok = scene_view(sbase).h->magic == kSceneMagic && scene_view(sbase).h->status == 0 &&
+                        (PA || !(B->flags & EHSS_BLOCK_PA));
         if (lane < kSmemBins) { A.count[lane] = 0; A.ledger[lane] = 0; }
         if (lane == 0) {
             const uint4 b0 = make_uint4(B->base[0], B->base[1], B->base[2], B->base[3]);
@@ -830,6 +863,18 @@ __global__ void __launch_bounds__(128, 8) k_blocks(const ehss_block* blocks, int
                         atomicAdd(&A.fp64, f);
                     }
                 }
+                // PA of a ray that is traced too: its first query has met a sphere for certain or missed every one
+                // for certain, unless a test was near-tangent (such a ray asks the any-hit query).  Disk rays start
+                // outside every sphere, where "meets" and "enters" agree.
+                if (PA && !RAYS && bounces == 0 && (__ldg(&B->flags) & EHSS_BLOCK_PA)) {
+                    bool blocked = k >= 0;
+                    if (W.grazing || W.overflow) {
+                        LocalStats pst;
+                        blocked = anyhit(S, L.o, L.d, -1, pst);
+                        if (COUNT) { W.box += pst.box; W.sphere += pst.sphere; }
+                    }
+                    if (blocked) atomicAdd(&A.pa, 1u);
+                }
                 if (k < 0 || bounces >= __ldg(&B->cap)) {
                     bool escaped = k < 0;
                     unsigned long long fx = 0;
@@ -862,7 +907,7 @@ __global__ void __launch_bounds__(128, 8) k_blocks(const ehss_block* blocks, int
                     ++bounces;
                     last_rank = k;
                     W.reset();
-                    if (!setup_ray(S.h, L.o, L.d, W.r, EXACT ? 0.0f : kWidenShortDisc)) W.error = true;   // bounce points lie within S
+                    if (!(EXACT ? setup_exact(S.h, L.o, L.d, W.r) : setup_ray(S.h, L.o, L.d, W.r, kWidenShortDisc))) W.error = true;   // bounce points lie within S
                     atomicAdd(&A.queries, 1u);
                     status = kTraverse;
                 }
@@ -893,7 +938,7 @@ __global__ void __launch_bounds__(128, 8) k_blocks(const ehss_block* blocks, int
 #pragma unroll
                             for (int i = 0; i < 3; ++i) { L.o[i] = ray.o[i]; L.d[i] = ray.d[i]; L.din[i] = ray.d[i]; }
                         }
-                        if (__ldg(&B->flags) & EHSS_BLOCK_PA) {
+                        if (PA && (__ldg(&B->flags) & EHSS_BLOCK_PA) && (RAYS || !(__ldg(&B->flags) & EHSS_BLOCK_EHSS))) {
                             LocalStats pst;
                             if (anyhit(S, L.o, L.d, -1, pst)) {
                                 atomicAdd(&A.pa, 1u);
@@ -906,7 +951,7 @@ __global__ void __launch_bounds__(128, 8) k_blocks(const ehss_block* blocks, int
                         last_rank = -1;
                         if (__ldg(&B->flags) & EHSS_BLOCK_EHSS) {
                             W.reset();
-                            if (!setup_ray(S.h, L.o, L.d, W.r, EXACT ? 0.0f : kWidenShortDisc)) W.error = true;
+                            if (!(EXACT ? setup_exact(S.h, L.o, L.d, W.r) : setup_ray(S.h, L.o, L.d, W.r, kWidenShortDisc))) W.error = true;
                             atomicAdd(&A.queries, 1u);
                             status = kTraverse;
                         }
@@ -1118,7 +1163,7 @@ __global__ void __launch_bounds__(128, kRayCtas) k_rays(const __grid_constant__ 
                 ++bounces;
                 last_rank = k;
                 W.reset();
-                if (!setup_ray(S.h, L.o, L.d, W.r, EXACT ? 0.0f : kWidenShortDisc)) { W.steps = -1; W.cur = kSentinel; }
+                if (!(EXACT ? setup_exact(S.h, L.o, L.d, W.r) : setup_ray(S.h, L.o, L.d, W.r, kWidenShortDisc))) { W.steps = -1; W.cur = kSentinel; }
                 atomicAdd(&A.queries, 1u);
                 status = kTraverse;
             }
@@ -1177,7 +1222,7 @@ __global__ void __launch_bounds__(128, kRayCtas) k_rays(const __grid_constant__ 
                         bounces = (int)count;
                         last_rank = last_id >= 0 ? S.rank[last_id] : -1;
                         W.reset();
-                        if (!setup_ray(S.h, L.o, L.d, W.r, EXACT ? 0.0f : kWidenShortDisc)) { W.steps = -1; W.cur = kSentinel; }
+                        if (!(EXACT ? setup_exact(S.h, L.o, L.d, W.r) : setup_ray(S.h, L.o, L.d, W.r, kWidenShortDisc))) { W.steps = -1; W.cur = kSentinel; }
                         atomicAdd(&A.queries, 1u);
                         status = kTraverse;
                     }
@@ -1277,7 +1322,7 @@ int launch_blocks(const ehss_block* blocks, int nb, int64_t chunk_first, int64_t
     const size_t smem_rays = smem + sizeof(double) * (size_t)L.block_threads;
     unsigned grid = (unsigned)(sm_count() * L.ctas_per_sm);
     int batch = L.resolve_batch > 0 ? L.resolve_batch : 1;
-    const bool count = (L.options & EHSS_LAUNCH_COUNT_TESTS) != 0;
+    const bool count = (L.options & EHSS_LAUNCH_COUNT_TESTS) != 0, pa = (L.options & EHSS_LAUNCH_NO_PA) == 0;
     // one launch per precision and ray kind present; each skips the other blocks' chunks
     const int mask = L.precisions ? L.precisions : 3;
     const int kinds = (L.options & EHSS_LAUNCH_RAY_BLOCKS) ? ((L.options & EHSS_LAUNCH_NO_DISK_BLOCKS) ? 2 : 3) : 1;
@@ -1293,17 +1338,19 @@ int launch_blocks(const ehss_block* blocks, int nb, int64_t chunk_first, int64_t
             }
             first = false;
             const int n_parts = sm_count() < kMaxWorkParts ? sm_count() : kMaxWorkParts;
-#define EHSS_LAUNCH_BLOCKS(E, C, R) \
-            k_blocks<E, C, R><<<grid, L.block_threads, R ? smem_rays : smem, stream>>>( \
+#define EHSS_LAUNCH_BLOCKS(E, C, R, P) \
+            k_blocks<E, C, R, P><<<grid, L.block_threads, R ? smem_rays : smem, stream>>>( \
                 blocks, nb, chunk_first, total_chunks, L.chunk_rays, batch, results, hist, ledger, work, n_parts, sdepth, \
                 residual, residual_capacity, residual_count)
+#define EHSS_PICK_PA(E, C, R) if (pa) EHSS_LAUNCH_BLOCKS(E, C, R, true); else EHSS_LAUNCH_BLOCKS(E, C, R, false)
+#define EHSS_PICK_COUNT(E, R) if (count) { EHSS_PICK_PA(E, true, R); } else { EHSS_PICK_PA(E, false, R); }
             if (exact) {
-                if (rays) { if (count) EHSS_LAUNCH_BLOCKS(true, true, true); else EHSS_LAUNCH_BLOCKS(true, false, true); }
-                else { if (count) EHSS_LAUNCH_BLOCKS(true, true, false); else EHSS_LAUNCH_BLOCKS(true, false, false); }
+                if (rays) { EHSS_PICK_COUNT(true, true) } else { EHSS_PICK_COUNT(true, false) }
             } else {
-                if (rays) { if (count) EHSS_LAUNCH_BLOCKS(false, true, true); else EHSS_LAUNCH_BLOCKS(false, false, true); }
-                else { if (count) EHSS_LAUNCH_BLOCKS(false, true, false); else EHSS_LAUNCH_BLOCKS(false, false, false); }
+                if (rays) { EHSS_PICK_COUNT(false, true) } else { EHSS_PICK_COUNT(false, false) }
             }
+#undef EHSS_PICK_COUNT
+#undef EHSS_PICK_PA
 #undef EHSS_LAUNCH_BLOCKS
             int rc = cuda_status(cudaGetLastError(), "blocks launch");
             if (rc) return rc;

@@ -340,9 +340,12 @@ typedef struct ehss_launch {
     int32_t reserved;         /* 0 */
 } ehss_launch;
 #define EHSS_LAUNCH_COUNT_TESTS 1   /* count box and sphere tests into the block stats (slower); a block
-                                       with EHSS_BLOCK_PA adds its any-hit tests to the same counters */
+                                       with EHSS_BLOCK_PA adds the any-hit tests it makes to the same counters
+                                       (none for a disk ray whose EHSS query decides PA) */
 #define EHSS_LAUNCH_RAY_BLOCKS 2    /* some blocks have EHSS_BLOCK_RAYS (adds a launch of that kernel instance) */
 #define EHSS_LAUNCH_NO_DISK_BLOCKS 4  /* with EHSS_LAUNCH_RAY_BLOCKS: every block has EHSS_BLOCK_RAYS */
+#define EHSS_LAUNCH_NO_PA 8           /* no block has EHSS_BLOCK_PA (one that has is counted in EHSS_STAT_ERRORS):
+                                         the kernel instance without the any-hit query, which needs fewer registers */
 
 /* Run all blocks in one persistent launch.  blocks_dev: device copy of the
  * prepared descriptors; results_dev[n_blocks], hist_dev/ledger_dev

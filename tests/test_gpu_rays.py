@@ -144,3 +144,47 @@ def test_any_hit_owners(n, pinned):
         blocked, box, sphere = index.query(src)
         assert blocked.dtype == bool and box + sphere > 0      # far origins test every atom and no box
         np.testing.assert_array_equal(blocked, tree.query(o, d, owners)[0])
+
+
+@pytest.mark.parametrize('scale', [1. - 3e-12, 1. + 1e-6, .5, 3.])
+def test_fp64_directions_off_unit_length(scale):
+    """The FP64 reject takes unit directions and is switched off for others."""
+    import torch
+    import ehss_b200 as eb
+    from ehss_b200 import _lib
+    c, r, o, d = _case(3000, 150, 13)
+    d = d * scale
+    scene = eb.Scene(c, r)
+    ref = O.trace_flat(c, r, o, d, cap=16)
+    P, D = torch.from_numpy(o).cuda(), torch.from_numpy(d).cuda()
+    last, b = torch.full((3000,), -1, device='cuda'), torch.zeros(3000, dtype=torch.int64, device='cuda')
+    esc, unres = (torch.zeros(3000, dtype=torch.uint8, device='cuda') for _ in range(2))
+    _lib.check(_lib.load().ehss_trace(scene.ptr, 3000, 16, 0, P.data_ptr(), D.data_ptr(), last.data_ptr(), b.data_ptr(),
+                                      esc.data_ptr(), unres.data_ptr(), None, None, torch.cuda.current_stream().cuda_stream))
+    for got, f in ((P, 'positions'), (D, 'outgoing'), (b, 'bounces'), (esc.bool(), 'escaped')):
+        np.testing.assert_array_equal(got.cpu().numpy(), ref[f], err_msg=f)
+
+
+@pytest.mark.parametrize('precision', [0, 1])
+@pytest.mark.parametrize('atoms,log2,exterior', [(1, 12, False), (3, 10, True), (300, 13, True), (2000, 12, False)])
+def test_pa_of_traced_blocks_equals_the_any_hit_query(precision, atoms, log2, exterior):
+    import ehss_b200 as eb
+    from ehss_b200 import _lib, workloads as W
+    from ehss_b200.blocks import BlockJob, BlockPlan
+    c, r = (np.zeros((1, 3)), np.array([2.7])) if atoms == 1 else W.globule(atoms, 17)[:2]
+    scene = eb.Scene(c, r, exterior=exterior)
+    kinds = ((True, True), (False, True), (True, False))
+    plan = BlockPlan([BlockJob(scene, log2, 5 + s, cap=32, precision=precision, ehss=e, pa=p) for s in range(3) for e, p in kinds])
+    plan.enqueue()
+    out = plan.collect()
+    for s in range(3):
+        both, only_pa, only_ehss = out[3 * s:3 * s + 3]
+        assert both['pa_blocked_rays'] == only_pa['pa_blocked_rays'] > 0
+        assert both['ehss_angstrom2'] == only_ehss['ehss_angstrom2']
+        assert both['collision_histogram'] == only_ehss['collision_histogram']
+    # the instance without the any-hit query reports a block that asks for it
+    wrong = BlockPlan([BlockJob(scene, log2, 5, precision=precision, pa=True)])
+    wrong.launch.options |= _lib.LAUNCH_NO_PA
+    wrong.enqueue()
+    with pytest.raises(_lib.EHSSDeviceError):
+        wrong.collect()
