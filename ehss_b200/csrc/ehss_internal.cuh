@@ -234,7 +234,7 @@ void sobol4_params(uint64_t seed, Sobol4Params* p);
 uint64_t build_workspace_bytes(int64_t N, int S);
 int build_scenes(int S, const double* const* xyz, const double* const* radii, const int64_t* n, int leaf_size,
                  void* const* scenes, const uint64_t* scene_bytes, void* workspace, uint64_t workspace_bytes,
-                 cudaStream_t stream, bool exterior = false);
+                 cudaStream_t stream, bool exterior = false, const double* centers = nullptr);
 int refit_scenes(int S, const double* const* xyz, const double* const* radii, const int64_t* n, void* const* scenes,
                  void* workspace, uint64_t workspace_bytes, cudaStream_t stream);
 // Rays whose results are copied to the host together (k_rays).

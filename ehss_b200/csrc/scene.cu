@@ -17,8 +17,6 @@
 //                  structure's centre box; key = structure << 31 | buried << 30
 //                  | code (buried only in the second pass of an exterior build)
 //   3. stable sort of (key, atom) pairs, so equal codes keep atom order:
-//                  per structure in one CTA (k_morton_segsort, steps 2-3 in one
-//                  launch) when every structure holds at most 8192 atoms, else
 //                  a device-wide LSD radix sort over the key's significant bits
 //                  (k_radix_count / k_radix_scan / k_radix_scatter, 8 bits a pass)
 //   4. k_karras    per internal node: Karras (2012) range / split search
@@ -30,6 +28,8 @@
 //                  by eps_box; subtrees of at most leaf_size atoms collapsed
 //                  into leaf references); per atom: FP32 and FP64 records in
 //                  leaf order, id maps.
+// Batches of structures of at most 8192 atoms run all of it in one launch,
+// one CTA a structure (k_build_small).
 // Exterior builds (EHSS_BUILD_EXTERIOR) then run k_exposure on that tree and
 // repeat steps 2-6 with the buried atoms sorted behind the exposed ones and
 // left out of the tree.
@@ -59,7 +59,8 @@ struct BuildDesc {
     int64_t n_active;          // atoms in the tree (exterior scenes: the exposed atoms)
     double cmin[3], cext[3];   // centre box relative to the scene centre (filled by k_stats)
     int32_t refit;             // 1: new coordinates for an existing full scene (tree kept)
-    int32_t pad;
+    int32_t centred;           // 1: center holds the centres' mean (summed in row order by the caller)
+    double center[3];
 };
 
 // Header status codes (0 = valid scene).
@@ -88,10 +89,11 @@ struct BuildWork {
 };
 
 // --------------------------------------------------------------------------
-__global__ void k_stats(BuildDesc* descs, int n_scenes) {
-    int s = blockIdx.x;
-    if (s >= n_scenes) return;
-    BuildDesc& D = descs[s];
+constexpr int kSumRows = 256;        // atoms of one chunk of the sequential coordinate sum
+
+// Header, centre, extents and input checks of one structure, by one CTA.
+// Returns false (to every thread) for a refit of a scene that cannot be refit.
+__device__ __forceinline__ bool scene_stats(BuildDesc& D) {
     SceneHeader* H = reinterpret_cast<SceneHeader*>(D.scene);
     const int64_t n = D.n;
     __shared__ double center[3];
@@ -110,7 +112,7 @@ __global__ void k_stats(BuildDesc* descs, int n_scenes) {
             bad = 0;
         }
         __syncthreads();
-        if (mismatch) return;
+        if (mismatch) return false;
     } else {
         // header: zeroed, then the layout offsets (the rest is filled below and by k_emit_nodes)
         if (threadIdx.x < sizeof(SceneHeader) / 4) reinterpret_cast<uint32_t*>(H)[threadIdx.x] = 0u;
@@ -122,20 +124,50 @@ __global__ void k_stats(BuildDesc* descs, int n_scenes) {
     }
     __syncthreads();
     // Sequential sum, one lane per coordinate: numpy's mean(axis=0) adds the
-    // rows in order and divides by n (ehss_state.py:46).
-    if (threadIdx.x < 3) {
-        int c = threadIdx.x;
+    // rows in order and divides by n (ehss_state.py:46).  The chain of dependent
+    // FP64 additions bounds it, so the coordinates come through shared memory
+    // (a chunk of the next while the last is added) and a lane's reads run
+    // ahead of its additions.
+    if (D.centred) {
+        if (threadIdx.x < 3) center[threadIdx.x] = D.center[threadIdx.x];
+    } else {
+        __shared__ double rows[2][kSumRows * 3];
         double acc = 0.;
-        int64_t i = 0;
-        for (; i + 8 <= n; i += 8) {         // loads ahead of the (sequential) sum
-            double v[8];
+        const int64_t total = 3 * n;
+        for (int64_t i = threadIdx.x; i < min((int64_t)(3 * kSumRows), total); i += blockDim.x) rows[0][i] = D.xyz[i];
+        __syncthreads();
+        for (int64_t base = 0, side = 0; base < total; base += 3 * kSumRows, side ^= 1) {
+            const int64_t next = base + 3 * kSumRows;
+            if (threadIdx.x >= 32 || blockDim.x <= 32)
+                for (int64_t i = threadIdx.x - (blockDim.x > 32 ? 32 : 0); i < min((int64_t)(3 * kSumRows), total - next);
+                     i += blockDim.x - (blockDim.x > 32 ? 32 : 0))
+                    rows[side ^ 1][i] = D.xyz[next + i];
+            if (threadIdx.x < 3) {
+                const double* v = rows[side] + threadIdx.x;
+                const int m = (int)min((int64_t)kSumRows, (total - base) / 3);
+                int i = 0;
+                if (m >= 16) {
+                    double x[8], y[8];
 #pragma unroll
-            for (int k = 0; k < 8; ++k) v[k] = D.xyz[(i + k) * 3 + c];
+                    for (int k = 0; k < 8; ++k) x[k] = v[3 * k];
+                    for (; i + 16 <= m; i += 16) {
 #pragma unroll
-            for (int k = 0; k < 8; ++k) acc = dadd(acc, v[k]);
+                        for (int k = 0; k < 8; ++k) y[k] = v[3 * (i + 8 + k)];
+#pragma unroll
+                        for (int k = 0; k < 8; ++k) acc = dadd(acc, x[k]);
+                        if (i + 24 <= m) {
+#pragma unroll
+                            for (int k = 0; k < 8; ++k) x[k] = v[3 * (i + 16 + k)];
+                        }
+#pragma unroll
+                        for (int k = 0; k < 8; ++k) acc = dadd(acc, y[k]);
+                    }
+                }
+                for (; i < m; ++i) acc = dadd(acc, v[3 * i]);
+            }
+            __syncthreads();
         }
-        for (; i < n; ++i) acc = dadd(acc, D.xyz[i * 3 + c]);
-        center[c] = ddiv(acc, (double)n);
+        if (threadIdx.x < 3) center[threadIdx.x] = ddiv(acc, (double)n);
     }
     // validation and radii extrema
     double rmax = 0.;
@@ -198,6 +230,12 @@ __global__ void k_stats(BuildDesc* descs, int n_scenes) {
             D.cext[c] = result[5 + c] + result[2 + c];
         }
     }
+    __syncthreads();
+    return true;
+}
+
+__global__ void k_stats(BuildDesc* descs, int n_scenes) {
+    if ((int)blockIdx.x < n_scenes) scene_stats(descs[blockIdx.x]);
 }
 
 __device__ __forceinline__ uint32_t spread10(uint32_t v) {
@@ -238,43 +276,7 @@ __global__ void k_morton(const BuildDesc* descs, const int32_t* atom_scene, int6
     vals[g] = (int32_t)i;
 }
 
-// Batches whose structures all hold at most kSegSortMax atoms: keys made and
-// sorted per structure by one CTA (stable block radix sort in shared memory),
-// one launch instead of the device-wide sort's several.  Keys never cross
-// structures, so the result equals the device-wide stable sort of k_morton's
-// keys element for element.  Two sizes: 256 x 8 keys (structures of at most
-// 2048 atoms) and 512 x 16 (8192).
-constexpr int kSegSortMax = 8192, kSegSortSmall = 2048;
-
-template <int THREADS, int ITEMS>
-__global__ void __launch_bounds__(THREADS, 1024 / THREADS) k_morton_segsort(const BuildDesc* descs,
-                                                                          const uint8_t* culled,
-                                                                          uint64_t* keys_out, int32_t* vals_out) {
-    using SegSort = cub::BlockRadixSort<uint32_t, THREADS, ITEMS, int32_t>;
-    static_assert(sizeof(typename SegSort::TempStorage) <= 48 * 1024, "segment sort storage fits static shared memory");
-    __shared__ typename SegSort::TempStorage temp;
-    const int s = blockIdx.x;
-    const BuildDesc& D = descs[s];
-    const SceneHeader* H = reinterpret_cast<const SceneHeader*>(D.scene);
-    const int n = D.n < THREADS * ITEMS ? (int)D.n : THREADS * ITEMS;     // the host sends no larger structure
-    uint32_t key[ITEMS];
-    int32_t val[ITEMS];
-#pragma unroll
-    for (int k = 0; k < ITEMS; ++k) {
-        const int i = threadIdx.x * ITEMS + k;              // blocked: item order = atom order
-        val[k] = i;
-        key[k] = i < n ? morton_key31(D, H, i, culled && D.exterior && culled[D.atom0 + i]) : 0xffffffffu;
-    }
-    SegSort(temp).Sort(key, val, 0, 32);
-#pragma unroll
-    for (int k = 0; k < ITEMS; ++k) {
-        const int j = threadIdx.x * ITEMS + k;
-        if (j < n) {
-            keys_out[D.atom0 + j] = ((uint64_t)s << 31) | key[k];
-            vals_out[D.atom0 + j] = val[k];
-        }
-    }
-}
+constexpr int kSegSortMax = 8192;      // batches of structures up to here build with one CTA each (k_build_small)
 
 // --------------------------------------------------------------------------
 // Device-wide stable LSD radix sort of (uint64 key, int32 value) pairs, for
@@ -397,62 +399,75 @@ static int radix_sort_pairs(uint64_t* keys_a, int32_t* vals_a, uint64_t* keys_b,
 }
 
 // Karras (2012), "Maximizing parallelism in the construction of BVHs,
-// octrees, and k-d trees": internal node i of a segment of n sorted keys.
-__device__ __forceinline__ int delta(const uint64_t* k, int64_t base, int n, int i, int j) {
-    if (j < 0 || j >= n) return -1;
-    uint64_t a = k[base + i], b = k[base + j];
-    if (a == b) return 64 + __clz((uint32_t)(i ^ j));
-    return __clzll(a ^ b);
+// octrees, and k-d trees": internal node i of a segment of sorted keys.
+// delta(x, y): length of the common prefix of keys x and y (their indices
+// extend equal keys), -1 when y lies outside the segment.
+struct KarrasNode {
+    int left, right, first, last;      // children: >= 0 internal node, < 0 ~leaf
+};
+
+template <typename Delta>
+__device__ __forceinline__ KarrasNode karras_node(Delta delta, int i) {
+    const int d = (delta(i, i + 1) - delta(i, i - 1)) >= 0 ? 1 : -1;
+    const int dmin = delta(i, i - d);
+    int lmax = 2;
+    while (delta(i, i + lmax * d) > dmin) lmax <<= 1;
+    int l = 0;
+    for (int t = lmax >> 1; t >= 1; t >>= 1)
+        if (delta(i, i + (l + t) * d) > dmin) l += t;
+    const int j = i + l * d;
+    const int dnode = delta(i, j);
+    int s = 0;
+    for (int t = (l + 1) >> 1;; t = (t + 1) >> 1) {
+        if (delta(i, i + (s + t) * d) > dnode) s += t;
+        if (t == 1) break;
+    }
+    const int gamma = i + s * d + (d < 0 ? d : 0);
+    KarrasNode k;
+    k.first = i < j ? i : j;
+    k.last = i < j ? j : i;
+    k.left = (k.first == gamma) ? ~gamma : gamma;
+    k.right = (k.last == gamma + 1) ? ~(gamma + 1) : gamma + 1;
+    return k;
+}
+
+// Structure owning global internal-node (or node) index g: last s with inner0 <= g.
+__device__ __forceinline__ int node_owner(const BuildDesc* descs, int n_scenes, int64_t g) {
+    int lo = 0, hi = n_scenes - 1;
+    while (lo < hi) {
+        int mid = (lo + hi + 1) >> 1;
+        if (descs[mid].inner0 <= g) lo = mid; else hi = mid - 1;
+    }
+    return lo;
 }
 
 __global__ void k_karras(const BuildDesc* descs, int n_scenes, int64_t I_total, const uint64_t* keys,
                          int32_t* inner_child, int32_t* inner_range, int32_t* parent_inner, int32_t* parent_leaf) {
     int64_t g = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (g >= I_total) return;
-    // structure owning inner node g: last s with inner0 <= g (binary search)
-    int lo = 0, hi = n_scenes - 1;
-    while (lo < hi) {
-        int mid = (lo + hi + 1) >> 1;
-        if (descs[mid].inner0 <= g) lo = mid; else hi = mid - 1;
-    }
-    const BuildDesc& D = descs[lo];
-    int n = (int)D.n_active;
-    int i = (int)(g - D.inner0);
+    const BuildDesc& D = descs[node_owner(descs, n_scenes, g)];
+    const int n = (int)D.n_active;
+    const int i = (int)(g - D.inner0);
     if (i >= n - 1) return;   // structures with one (active) atom own no internal node
-    int64_t base = D.atom0;
-    int d = (delta(keys, base, n, i, i + 1) - delta(keys, base, n, i, i - 1)) >= 0 ? 1 : -1;
-    int dmin = delta(keys, base, n, i, i - d);
-    int lmax = 2;
-    while (delta(keys, base, n, i, i + lmax * d) > dmin) lmax <<= 1;
-    int l = 0;
-    for (int t = lmax >> 1; t >= 1; t >>= 1)
-        if (delta(keys, base, n, i, i + (l + t) * d) > dmin) l += t;
-    int j = i + l * d;
-    int dnode = delta(keys, base, n, i, j);
-    int s = 0;
-    int span = l;
-    for (int t = (span + 1) >> 1;; t = (t + 1) >> 1) {
-        if (delta(keys, base, n, i, i + (s + t) * d) > dnode) s += t;
-        if (t == 1) break;
-    }
-    int gamma = i + s * d + (d < 0 ? d : 0);
-    int first = i < j ? i : j, last = i < j ? j : i;
-    int64_t gi = D.inner0 + i;
-    inner_range[2 * gi] = first;
-    inner_range[2 * gi + 1] = last;
-    int left = (first == gamma) ? ~gamma : gamma;
-    int right = (last == gamma + 1) ? ~(gamma + 1) : gamma + 1;
-    inner_child[2 * gi] = left;
-    inner_child[2 * gi + 1] = right;
-    if (left < 0) parent_leaf[base + gamma] = i; else parent_inner[D.inner0 + left] = i;
-    if (right < 0) parent_leaf[base + gamma + 1] = i; else parent_inner[D.inner0 + right] = i;
-    if (i == 0) parent_inner[gi] = -1;
+    const int64_t base = D.atom0;
+    const KarrasNode k = karras_node([&](int x, int y) -> int {
+        if (y < 0 || y >= n) return -1;
+        const uint64_t a = keys[base + x], b = keys[base + y];
+        return a == b ? 64 + __clz((uint32_t)(x ^ y)) : __clzll(a ^ b);
+    }, i);
+    inner_range[2 * g] = k.first;
+    inner_range[2 * g + 1] = k.last;
+    inner_child[2 * g] = k.left;
+    inner_child[2 * g + 1] = k.right;
+    if (k.left < 0) parent_leaf[base + ~k.left] = i; else parent_inner[D.inner0 + k.left] = i;
+    if (k.right < 0) parent_leaf[base + ~k.right] = i; else parent_inner[D.inner0 + k.right] = i;
+    if (i == 0) parent_inner[g] = -1;
 }
 
-__device__ __forceinline__ void atom_box(const BuildDesc& D, const SceneHeader* H, int64_t atom, float* b) {
-    double r = D.radii[atom];
+__device__ __forceinline__ void atom_box(const double* xyz, const double* radii, const double* center, int64_t atom, float* b) {
+    const double r = radii[atom];
     for (int c = 0; c < 3; ++c) {
-        double rel = D.xyz[atom * 3 + c] - H->center[c];
+        const double rel = xyz[atom * 3 + c] - center[c];
         b[c] = __double2float_rd(rel - r);
         b[3 + c] = __double2float_ru(rel + r);
     }
@@ -466,7 +481,7 @@ __global__ void k_refit(const BuildDesc* descs, const int32_t* atom_scene, int64
     const BuildDesc& D = descs[atom_scene[g]];
     const SceneHeader* H = reinterpret_cast<const SceneHeader*>(D.scene);
     float b[6];
-    atom_box(D, H, vals_sorted[g], b);
+    atom_box(D.xyz, D.radii, H->center, vals_sorted[g], b);
     for (int k = 0; k < 6; ++k) leaf_box[6 * g + k] = b[k];
     if (D.n_active == 1 || g - D.atom0 >= D.n_active) return;    // no tree above, or a buried atom
     int node = parent_leaf[g];
@@ -518,56 +533,44 @@ __device__ __forceinline__ void write_node4(float4* nodes, int64_t i, const floa
     nd[7] = make_float4(0.f, 0.f, 0.f, 0.f);
 }
 
-__global__ void k_emit_nodes(const BuildDesc* descs, int n_scenes, int64_t I_total, const int32_t* inner_child,
-                             const int32_t* inner_range, const float* inner_box, const float* leaf_box,
-                             const int32_t* inner_height) {
-    int64_t g = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    // one extra thread per structure handles the single-leaf case (n <= leaf_size)
-    if (g >= I_total + n_scenes) return;
-    if (g >= I_total) {
-        const BuildDesc& D = descs[g - I_total];
-        SceneHeader* H = reinterpret_cast<SceneHeader*>(D.scene);
-        H->n_active = (int32_t)D.n_active;
-        H->exterior = D.exterior;
-        if (D.n_active > D.leaf_size) {
-            H->depth = inner_height[D.inner0];
-            H->n_nodes = (int32_t)(D.n_active - 1);
-            return;
-        }
-        // whole structure in one leaf below a single node
-        float4* nodes = reinterpret_cast<float4*>(D.scene + H->off_nodes);
-        float u[1][6] = {{CUDART_INF_F, CUDART_INF_F, CUDART_INF_F, -CUDART_INF_F, -CUDART_INF_F, -CUDART_INF_F}};
-        for (int64_t a = 0; a < D.n_active; ++a)
-            for (int k = 0; k < 3; ++k) {
-                u[0][k] = fminf(u[0][k], leaf_box[6 * (D.atom0 + a) + k]);
-                u[0][3 + k] = fmaxf(u[0][3 + k], leaf_box[6 * (D.atom0 + a) + 3 + k]);
-            }
-        int ref = ~((0 << kLeafBits) | (int)(D.n_active - 1));
-        write_node4(nodes, 0, u, &ref, 1, H->eps_box);
-        H->depth = 1;
-        H->n_nodes = 1;
+// Header fields of a finished tree (depth: the binary tree's height), and the
+// single node of a structure that fits one leaf.  leaf_box: the structure's own.
+__device__ __forceinline__ void finish_header(const BuildDesc& D, SceneHeader* H, const float* leaf_box, int depth) {
+    H->n_active = (int32_t)D.n_active;
+    H->exterior = D.exterior;
+    if (D.n_active > D.leaf_size) {
+        H->depth = depth;
+        H->n_nodes = (int32_t)(D.n_active - 1);
         return;
     }
-    int lo = 0, hi = n_scenes - 1;
-    while (lo < hi) {
-        int mid = (lo + hi + 1) >> 1;
-        if (descs[mid].inner0 <= g) lo = mid; else hi = mid - 1;
-    }
-    const BuildDesc& D = descs[lo];
-    int i = (int)(g - D.inner0);
-    if (i >= D.n_active - 1 || D.n_active <= D.leaf_size) return;
-    SceneHeader* H = reinterpret_cast<SceneHeader*>(D.scene);
+    // whole structure in one leaf below a single node
+    float4* nodes = reinterpret_cast<float4*>(D.scene + H->off_nodes);
+    float u[1][6] = {{CUDART_INF_F, CUDART_INF_F, CUDART_INF_F, -CUDART_INF_F, -CUDART_INF_F, -CUDART_INF_F}};
+    for (int64_t a = 0; a < D.n_active; ++a)
+        for (int k = 0; k < 3; ++k) {
+            u[0][k] = fminf(u[0][k], leaf_box[6 * a + k]);
+            u[0][3 + k] = fmaxf(u[0][3 + k], leaf_box[6 * a + 3 + k]);
+        }
+    int ref = ~((0 << kLeafBits) | (int)(D.n_active - 1));
+    write_node4(nodes, 0, u, &ref, 1, H->eps_box);
+    H->depth = 1;
+    H->n_nodes = 1;
+}
+
+// 4-wide record i from binary node i (arrays: the structure's own).
+__device__ __forceinline__ void emit_node(const BuildDesc& D, const SceneHeader* H, int i, const int32_t* inner_child,
+                                          const int32_t* inner_range, const float* inner_box, const float* leaf_box) {
     float4* nodes = reinterpret_cast<float4*>(D.scene + H->off_nodes);
     // slot of a binary child: leaf reference when it is an atom or a subtree
     // of at most leaf_size atoms, else the node index (expanded once more)
     auto classify = [&](int c, int& ref, const float*& box) -> bool {   // true: expandable internal node
         if (c < 0) {
-            box = leaf_box + 6 * (D.atom0 + ~c);
+            box = leaf_box + 6 * (int64_t)~c;
             ref = ~((~c) << kLeafBits);
             return false;
         }
-        box = inner_box + 6 * (D.inner0 + c);
-        int first = inner_range[2 * (D.inner0 + c)], last = inner_range[2 * (D.inner0 + c) + 1];
+        box = inner_box + 6 * (int64_t)c;
+        int first = inner_range[2 * (int64_t)c], last = inner_range[2 * (int64_t)c + 1];
         int count = last - first + 1;
         if (count <= D.leaf_size) { ref = ~((first << kLeafBits) | (count - 1)); return false; }
         ref = c;
@@ -577,7 +580,7 @@ __global__ void k_emit_nodes(const BuildDesc* descs, int n_scenes, int64_t I_tot
     float boxes[4][6];
     int n = 0;
     for (int side = 0; side < 2; ++side) {
-        int c = inner_child[2 * g + side];
+        int c = inner_child[2 * (int64_t)i + side];
         int ref;
         const float* box;
         if (!classify(c, ref, box)) {
@@ -587,7 +590,7 @@ __global__ void k_emit_nodes(const BuildDesc* descs, int n_scenes, int64_t I_tot
             continue;
         }
         for (int side2 = 0; side2 < 2; ++side2) {          // grandchildren
-            int gc = inner_child[2 * (D.inner0 + c) + side2];
+            int gc = inner_child[2 * (int64_t)c + side2];
             int ref2;
             const float* box2;
             classify(gc, ref2, box2);
@@ -599,13 +602,8 @@ __global__ void k_emit_nodes(const BuildDesc* descs, int n_scenes, int64_t I_tot
     write_node4(nodes, i, boxes, refs, n, H->eps_box);
 }
 
-__global__ void k_emit_atoms(const BuildDesc* descs, const int32_t* atom_scene, int64_t N, const int32_t* vals_sorted) {
-    int64_t g = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (g >= N) return;
-    const BuildDesc& D = descs[atom_scene[g]];
-    SceneHeader* H = reinterpret_cast<SceneHeader*>(D.scene);
-    int64_t j = g - D.atom0;               // leaf-order position
-    int64_t a = vals_sorted[g];            // input atom id
+// Records of the atom in leaf-order slot j, input atom a.
+__device__ __forceinline__ void emit_atom(const BuildDesc& D, const SceneHeader* H, int64_t j, int64_t a) {
     float4* atoms = reinterpret_cast<float4*>(D.scene + H->off_atoms);
     double4* atoms64 = reinterpret_cast<double4*>(D.scene + H->off_atoms64);
     int32_t* ids = reinterpret_cast<int32_t*>(D.scene + H->off_ids);
@@ -616,6 +614,192 @@ __global__ void k_emit_atoms(const BuildDesc* descs, const int32_t* atom_scene, 
     atoms64[j] = make_double4(x, y, z, r);
     ids[j] = (int32_t)a;
     rank[a] = (int32_t)j;
+}
+
+// All records of a batch: threads 0 .. N-1 the atoms, then the internal nodes,
+// then one a structure for its header.
+__global__ void k_emit(const BuildDesc* descs, int n_scenes, const int32_t* atom_scene, int64_t N, int64_t I_total,
+                       const int32_t* vals_sorted, const int32_t* inner_child, const int32_t* inner_range,
+                       const float* inner_box, const float* leaf_box, const int32_t* inner_height) {
+    int64_t g = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    if (g < N) {
+        const BuildDesc& D = descs[atom_scene[g]];
+        emit_atom(D, reinterpret_cast<const SceneHeader*>(D.scene), g - D.atom0, vals_sorted[g]);
+        return;
+    }
+    g -= N;
+    if (g < I_total) {
+        const BuildDesc& D = descs[node_owner(descs, n_scenes, g)];
+        const int i = (int)(g - D.inner0);
+        if (i >= D.n_active - 1 || D.n_active <= D.leaf_size) return;
+        emit_node(D, reinterpret_cast<const SceneHeader*>(D.scene), i, inner_child + 2 * D.inner0, inner_range + 2 * D.inner0,
+                  inner_box + 6 * D.inner0, leaf_box + 6 * D.atom0);
+        return;
+    }
+    g -= I_total;
+    if (g >= n_scenes) return;
+    const BuildDesc& D = descs[g];
+    finish_header(D, reinterpret_cast<SceneHeader*>(D.scene), leaf_box + 6 * D.atom0,
+                  D.n_active > 1 ? inner_height[D.inner0] : 0);
+}
+
+// --------------------------------------------------------------------------
+// Batches whose structures all hold at most kSegSortMax atoms: one CTA makes
+// one structure's tree in one launch (a launch a pass: the full tree, and for
+// exterior scenes the tree over the exposed atoms after k_exposure), and k_emit
+// writes the records on all SMs.  The phases are those of the device-wide path
+// -- statistics, Morton keys and their stable sort, Karras hierarchy, bottom-up
+// boxes -- with __syncthreads between them instead of launches; the sorted
+// keys, parent links, arrival flags and (where they fit) the node boxes lie in
+// shared memory, so a step of the bottom-up walk costs shared-memory latencies
+// and a CTA-scope fence instead of device-scope ones.  The scenes are the
+// device-wide path's byte for byte.
+// Bound by latency: of the full tree of 5000 atoms (160 us) the sequential
+// coordinate sum takes 30 %, the sort 25 %, the walk up 35 %.  Both passes with
+// k_emit: 72 us for 650 atoms (160 us as eleven launches), 163 us for 5000
+// (260), 355 us for 256 structures of 20-5000 atoms (435).
+// THREADS x ITEMS is the largest structure of the instance; smaller ones sort
+// with half or a quarter of the items, as they are.
+// --------------------------------------------------------------------------
+template <int THREADS, int ITEMS>
+struct SmallBuild {
+    static constexpr int kMax = THREADS * ITEMS;
+    template <int I>
+    using Sort = cub::BlockRadixSort<uint32_t, THREADS, I, int32_t, 5>;
+    union Scratch {
+        typename Sort<ITEMS>::TempStorage sort;
+        typename Sort<(ITEMS > 1 ? ITEMS / 2 : 1)>::TempStorage half;
+        typename Sort<(ITEMS > 3 ? ITEMS / 4 : 1)>::TempStorage quarter;
+        struct {
+            uint16_t parent_inner[kMax], parent_leaf[kMax];
+            uint8_t height[kMax];
+            unsigned first[kMax];      // the child that arrived first: leaf flag << 31 | index
+        } tree;
+    };
+    Scratch scratch;
+    uint16_t atom[kMax];
+    uint32_t key[kMax];                // then, from here on, the node boxes if the launch has room for them
+    static size_t bytes(int64_t boxes) { return sizeof(SmallBuild) - sizeof(key) + std::max(sizeof(key), 24 * (size_t)boxes); }
+};
+constexpr int kNoParent = 0xffff;
+constexpr unsigned kNobody = 0xffffffffu, kIsLeaf = 0x80000000u;
+
+template <int THREADS, int I, typename Temp>
+__device__ __forceinline__ void small_sort(const BuildDesc& D, const SceneHeader* H, const uint8_t* culled, Temp& temp,
+                                           uint32_t* key_out, uint16_t* atom_out) {
+    uint32_t key[I];
+    int32_t val[I];
+    const int n = (int)D.n;
+#pragma unroll
+    for (int k = 0; k < I; ++k) {
+        const int i = threadIdx.x * I + k;                  // blocked: item order = atom order
+        val[k] = i;
+        // padding sorts behind every key: the largest one, and behind its equals by the stable order
+        key[k] = i < n ? morton_key31(D, H, i, culled && D.exterior && culled[D.atom0 + i]) : 0x7fffffffu;
+    }
+    cub::BlockRadixSort<uint32_t, THREADS, I, int32_t, 5>(temp).Sort(key, val, 0, 31);
+#pragma unroll
+    for (int k = 0; k < I; ++k) {
+        const int j = threadIdx.x * I + k;
+        if (j < n) {
+            key_out[j] = key[k];
+            atom_out[j] = (uint16_t)val[k];
+        }
+    }
+}
+
+template <int THREADS, int ITEMS>
+__global__ void __launch_bounds__(THREADS) k_build_small(BuildDesc* descs, int32_t* atom_scene, const uint8_t* culled,
+                                                         int32_t* inner_child, int32_t* inner_range, float* inner_box,
+                                                         float* leaf_box, int32_t* inner_height, int32_t* vals_out,
+                                                         int smem_boxes) {
+    extern __shared__ __align__(16) unsigned char small_smem[];
+    SmallBuild<THREADS, ITEMS>& B = *reinterpret_cast<SmallBuild<THREADS, ITEMS>*>(small_smem);
+    BuildDesc& D = descs[blockIdx.x];
+    SceneHeader* const H = reinterpret_cast<SceneHeader*>(D.scene);
+    const int n = (int)D.n;
+    if (culled) {
+        // a structure whose atoms all tested buried (impossible for a bounded union: its boundary
+        // lies on some exposed sphere) falls back to the full tree
+        if (threadIdx.x == 0 && D.n_active < 1) { D.n_active = n; D.exterior = 0; }
+        __syncthreads();
+    } else {
+        scene_stats(D);
+        for (int i = threadIdx.x; i < n; i += THREADS) atom_scene[D.atom0 + i] = blockIdx.x;
+    }
+    if (n > THREADS * ITEMS) return;                        // the host sends no larger structure
+    // ---- sorted keys ----
+    if (ITEMS > 3 && n <= THREADS * (ITEMS / 4))
+        small_sort<THREADS, (ITEMS > 3 ? ITEMS / 4 : 1)>(D, H, culled, B.scratch.quarter, B.key, B.atom);
+    else if (ITEMS > 1 && n <= THREADS * (ITEMS / 2))
+        small_sort<THREADS, (ITEMS > 1 ? ITEMS / 2 : 1)>(D, H, culled, B.scratch.half, B.key, B.atom);
+    else
+        small_sort<THREADS, ITEMS>(D, H, culled, B.scratch.sort, B.key, B.atom);
+    __syncthreads();
+    auto& T = B.scratch.tree;
+    const int m = (int)D.n_active;                          // atoms of the tree: the first m in leaf order
+    for (int i = threadIdx.x; i < m - 1; i += THREADS) T.first[i] = kNobody;
+    // ---- hierarchy ----
+    int32_t* const child = inner_child + 2 * D.inner0;
+    int32_t* const range = inner_range + 2 * D.inner0;
+    float* const ibox = inner_box + 6 * D.inner0;
+    float* const lbox = leaf_box + 6 * D.atom0;
+    for (int i = threadIdx.x; i < m - 1; i += THREADS) {
+        const KarrasNode k = karras_node([&](int x, int y) -> int {
+            if (y < 0 || y >= m) return -1;
+            const uint32_t p = B.key[x], q = B.key[y];
+            return p == q ? 64 + __clz((uint32_t)(x ^ y)) : __clz(p ^ q);
+        }, i);
+        child[2 * i] = k.left;
+        child[2 * i + 1] = k.right;
+        range[2 * i] = k.first;
+        range[2 * i + 1] = k.last;
+        if (k.left < 0) T.parent_leaf[~k.left] = (uint16_t)i; else T.parent_inner[k.left] = (uint16_t)i;
+        if (k.right < 0) T.parent_leaf[~k.right] = (uint16_t)i; else T.parent_inner[k.right] = (uint16_t)i;
+        if (i == 0) T.parent_inner[0] = kNoParent;
+    }
+    __syncthreads();
+    // ---- leaf order, atom boxes and the way up: the second child to arrive at a node unites the boxes; the first
+    // leaves its name there, so a step reads one box and takes one shared-memory exchange ----
+    float* const box = m - 1 <= smem_boxes ? reinterpret_cast<float*>(B.key) : nullptr;    // the keys are done with
+    // in registers: the stores below may alias the descriptor and the header as far as the compiler knows
+    const double* const xyz = D.xyz;
+    const double* const radii = D.radii;
+    const double center[3] = {H->center[0], H->center[1], H->center[2]};
+    int32_t* const vals = vals_out + D.atom0;
+    int32_t* const root_height = inner_height + D.inner0;
+    for (int j = threadIdx.x; j < n; j += THREADS) {
+        const int a = B.atom[j];
+        vals[j] = a;
+        float u[6];
+        atom_box(xyz, radii, center, a, u);
+        for (int k = 0; k < 6; ++k) lbox[6 * j + k] = u[k];
+        if (m == 1 || j >= m) continue;                     // no tree above, or a buried atom
+        int node = T.parent_leaf[j], h = 0;
+        unsigned self = kIsLeaf | (unsigned)j;
+        // a walk longer than any LBVH depth (Morton bits + duplicate bits) means a malformed link
+        for (int hops = 0; node != kNoParent && hops < 128; ++hops) {
+            __threadfence_block();
+            const unsigned other = atomicExch(&T.first[node], self);
+            if (other == kNobody) break;
+            __threadfence_block();
+            const int c = (int)(other & ~kIsLeaf);
+            const float* src = other & kIsLeaf ? lbox + 6 * c : box ? box + 6 * c : ibox + 6 * c;
+            for (int k = 0; k < 3; ++k) {
+                u[k] = fminf(u[k], src[k]);
+                u[3 + k] = fmaxf(u[3 + k], src[3 + k]);
+            }
+            h = max(h, other & kIsLeaf ? 0 : (int)T.height[c]) + 1;
+            for (int k = 0; k < 6; ++k) {
+                if (box) box[6 * node + k] = u[k];
+                ibox[6 * node + k] = u[k];
+            }
+            T.height[node] = (uint8_t)h;
+            if (node == 0) *root_height = h;
+            self = (unsigned)node;
+            node = T.parent_inner[node];
+        }
+    }
 }
 
 __global__ void k_fill_scene_index(const BuildDesc* descs, int n_scenes, int32_t* atom_scene) {
@@ -663,18 +847,8 @@ __global__ void k_refit_atoms(const BuildDesc* descs, const int32_t* atom_scene,
                            __double2float_rn(z - H->center[2]), __double2float_rn(r));
     atoms64[j] = make_double4(x, y, z, r);
     float b[6];
-    atom_box(D, H, a, b);
+    atom_box(D.xyz, D.radii, H->center, a, b);
     for (int k = 0; k < 6; ++k) leaf_box[6 * g + k] = b[k];
-}
-
-// Structure owning global node index g (last s with inner0 <= g).
-__device__ __forceinline__ int node_owner(const BuildDesc* descs, int n_scenes, int64_t g) {
-    int lo = 0, hi = n_scenes - 1;
-    while (lo < hi) {
-        int mid = (lo + hi + 1) >> 1;
-        if (descs[mid].inner0 <= g) lo = mid; else hi = mid - 1;
-    }
-    return lo;
 }
 
 __global__ void k_node_links(const BuildDesc* descs, int n_scenes, int64_t nodes_total, int32_t* parent,
@@ -1244,9 +1418,36 @@ uint64_t build_workspace_bytes(int64_t N, int S) {
     return b + 256;
 }
 
+// k_build_small, the instance for structures of at most max_n atoms.  Node
+// boxes go to shared memory where an SM holds `ctas` such CTAs.
+template <int THREADS, int ITEMS>
+static int launch_small(int S, int64_t max_n, int ctas, const BuildWork& W, const uint8_t* culled, cudaStream_t stream) {
+    using B = SmallBuild<THREADS, ITEMS>;
+    constexpr int kSmemPerSM = 227 * 1024, kStatic = 16 * 1024;     // scene_stats' static arrays, rounded up
+    int boxes = (int)max_n - 1;
+    if ((int64_t)(B::bytes(boxes) + kStatic) * ctas > kSmemPerSM) boxes = 0;
+    const int smem = (int)B::bytes(boxes);
+    // held per device and context, so set on each call (a limit, not an allocation)
+    const int rc = cuda_status(cudaFuncSetAttribute(k_build_small<THREADS, ITEMS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                    smem), "LBVH build");
+    if (rc) return rc;
+    k_build_small<THREADS, ITEMS><<<S, THREADS, smem, stream>>>(W.descs, W.atom_scene, culled, W.inner_child, W.inner_range,
+                                                                W.inner_box, W.leaf_box, W.inner_height, W.vals_out, boxes);
+    return cuda_status(cudaGetLastError(), "LBVH build launch");
+}
+
+static int launch_build_small(int S, int64_t max_n, const BuildWork& W, const uint8_t* culled, cudaStream_t stream) {
+    // one CTA an SM while every structure has an SM to itself, else two
+    const bool few = S <= sm_count();
+    if (max_n <= 1024) return launch_small<512, 2>(S, max_n, few ? 1 : 3, W, culled, stream);
+    if (max_n <= 2048) return few ? launch_small<1024, 2>(S, max_n, 1, W, culled, stream)
+                                  : launch_small<512, 4>(S, max_n, 2, W, culled, stream);
+    return few ? launch_small<1024, 8>(S, max_n, 1, W, culled, stream) : launch_small<512, 16>(S, max_n, 2, W, culled, stream);
+}
+
 int build_scenes(int S, const double* const* xyz, const double* const* radii, const int64_t* n, int leaf_size,
                  void* const* scenes, const uint64_t* scene_bytes, void* workspace, uint64_t workspace_bytes,
-                 cudaStream_t stream, bool exterior) {
+                 cudaStream_t stream, bool exterior, const double* centers) {
     if (S < 1) { set_error("at least one structure required"); return EHSS_ERR_VALUE; }
     if (leaf_size < 1 || leaf_size > kMaxLeaf) { set_error("leaf_size must be 1..%d", kMaxLeaf); return EHSS_ERR_VALUE; }
     int64_t N = 0, I = 0, max_n = 0;
@@ -1274,7 +1475,9 @@ int build_scenes(int S, const double* const* xyz, const double* const* radii, co
         D.xyz = xyz[s]; D.radii = radii[s]; D.scene = (char*)scenes[s];
         D.n = n[s]; D.atom0 = N; D.inner0 = I; D.leaf_size = leaf_size; D.exterior = exterior ? 1 : 0;
         D.n_active = n[s];
-        D.refit = 0; D.pad = 0;
+        D.refit = 0;
+        D.centred = centers != nullptr;
+        for (int c = 0; c < 3; ++c) D.center[c] = centers ? centers[3 * s + c] : 0.;
         if (n[s] > max_n) max_n = n[s];
         N += n[s];
         I += n[s] - 1;
@@ -1322,28 +1525,26 @@ int build_scenes(int S, const double* const* xyz, const double* const* radii, co
 
     const int T = 256;
     auto blocks = [&](int64_t count) { return (unsigned)((count + T - 1) / T); };
-    k_fill_scene_index<<<S, 256, 0, stream>>>(W.descs, S, W.atom_scene);
-    k_stats<<<S, 256, 0, stream>>>(W.descs, S);
+    const bool small = max_n <= kSegSortMax;
+    if (!small) {
+        k_fill_scene_index<<<S, 256, 0, stream>>>(W.descs, S, W.atom_scene);
+        k_stats<<<S, 256, 0, stream>>>(W.descs, S);
+    }
     int end_bit = 31;
     while ((1ll << (end_bit - 31)) < S) ++end_bit;
-    const bool segsort = max_n <= kSegSortMax;
     // one pass: Morton keys -> sort -> Karras hierarchy -> refit -> node and atom records
     auto tree_pass = [&](const uint8_t* culled) -> int {
         int r;
-        if (segsort) {
-            if (max_n <= kSegSortSmall)
-                k_morton_segsort<256, 8><<<S, 256, 0, stream>>>(W.descs, culled, W.keys_out, W.vals_out);
-            else
-                k_morton_segsort<512, 16><<<S, 512, 0, stream>>>(W.descs, culled, W.keys_out, W.vals_out);
-            r = cuda_status(cudaGetLastError(), "LBVH key sort");
+        if (small) {
+            r = launch_build_small(S, max_n, W, culled, stream);
+            if (r) return r;
         } else {
-            // the keys start in the buffer from which an odd or even number of passes ends in keys_out
-            const bool odd = radix_passes(end_bit) % 2 != 0;
-            k_morton<<<blocks(N), T, 0, stream>>>(W.descs, W.atom_scene, N, culled, odd ? W.keys_in : W.keys_out,
-                                                  odd ? W.vals_in : W.vals_out);
-            r = radix_sort_pairs(W.keys_in, W.vals_in, W.keys_out, W.vals_out, N, end_bit, W.radix_counts,
-                                 W.radix_offsets, stream);
-        }
+        // the keys start in the buffer from which an odd or even number of passes ends in keys_out
+        const bool odd = radix_passes(end_bit) % 2 != 0;
+        k_morton<<<blocks(N), T, 0, stream>>>(W.descs, W.atom_scene, N, culled, odd ? W.keys_in : W.keys_out,
+                                              odd ? W.vals_in : W.vals_out);
+        r = radix_sort_pairs(W.keys_in, W.vals_in, W.keys_out, W.vals_out, N, end_bit, W.radix_counts,
+                             W.radix_offsets, stream);
         if (r) return r;
         // parent links start at -1 so that a missing link ends a refit walk
         r = cuda_status(cudaMemsetAsync(W.parent_leaf, 0xff, 4ull * N, stream), "LBVH parent reset");
@@ -1357,9 +1558,9 @@ int build_scenes(int S, const double* const* xyz, const double* const* radii, co
         }
         k_refit<<<blocks(N), T, 0, stream>>>(W.descs, W.atom_scene, N, W.vals_out, W.inner_child, W.parent_inner,
                                              W.parent_leaf, W.inner_box, W.leaf_box, W.inner_height, W.arrivals);
-        k_emit_nodes<<<blocks(I + S), T, 0, stream>>>(W.descs, S, I, W.inner_child, W.inner_range, W.inner_box,
-                                                      W.leaf_box, W.inner_height);
-        k_emit_atoms<<<blocks(N), T, 0, stream>>>(W.descs, W.atom_scene, N, W.vals_out);
+        }
+        k_emit<<<blocks(N + I + S), T, 0, stream>>>(W.descs, S, W.atom_scene, N, I, W.vals_out, W.inner_child, W.inner_range,
+                                                    W.inner_box, W.leaf_box, W.inner_height);
         return cuda_status(cudaGetLastError(), "LBVH build launch");
     };
     rc = tree_pass(nullptr);
@@ -1379,7 +1580,7 @@ int build_scenes(int S, const double* const* xyz, const double* const* radii, co
         unsigned grid = (unsigned)(want < cap ? want : cap);
         k_exposure<<<grid, 32 * kExposureWarps, 0, stream>>>(W.descs, W.atom_scene, N, W.culled);
     }
-    k_finish_exposure<<<(S + 127) / 128, 128, 0, stream>>>(W.descs, S);
+    if (!small) k_finish_exposure<<<(S + 127) / 128, 128, 0, stream>>>(W.descs, S);
     rc = cuda_status(cudaGetLastError(), "exposure launch");
     if (rc) return rc;
     return tree_pass(W.culled);
