@@ -68,22 +68,15 @@ class BatchScenes:
         # pinned host staging, one contiguous copy per array
         self.h_xyz = t.empty(N * 3, dtype=t.float64, pin_memory=True)
         self.h_r = t.empty(N, dtype=t.float64, pin_memory=True)
-        hx, hr = self.h_xyz.numpy(), self.h_r.numpy()
-        radii = []
-        for (c, r), a0, n in zip(structures, self.atom0, self.n_atoms):
-            c = np.ascontiguousarray(c, dtype=np.float64); r = np.ascontiguousarray(r, dtype=np.float64)
-            if c.shape != (n, 3) or not np.isfinite(c).all() or not np.isfinite(r).all() or np.any(r <= 0):
-                raise ValueError('Finite centers (N,3) and positive finite radii required.')
-            hx[3 * a0:3 * (a0 + n)] = c.ravel()
-            hr[a0:a0 + n] = r
-            radii.append(enclosing_radius(c, r))
+        radii = self._stage(structures, 'Finite centers (N,3) and positive finite radii required.')
         self.d_xyz = t.empty(N * 3, dtype=t.float64, device=self.device)
         self.d_r = t.empty(N, dtype=t.float64, device=self.device)
-        sizes = []
-        for n in self.n_atoms:
+        size_of = {}
+        for n in set(self.n_atoms.tolist()):
             sb, wb = ct.c_uint64(), ct.c_uint64()
-            _lib.check(lib.ehss_scene_bytes(int(n), int(leaf_size), ct.byref(sb), ct.byref(wb)), 'scene size')
-            sizes.append(sb.value)
+            _lib.check(lib.ehss_scene_bytes(n, int(leaf_size), ct.byref(sb), ct.byref(wb)), 'scene size')
+            size_of[n] = sb.value
+        sizes = [size_of[n] for n in self.n_atoms.tolist()]
         offs = np.concatenate([[0], np.cumsum(sizes)[:-1]]).astype(np.int64)
         self.scene_buf = t.empty(int(sum(sizes)) + 256, dtype=t.uint8, device=self.device)
         base = (self.scene_buf.data_ptr() + 255) & ~255
@@ -114,9 +107,10 @@ class BatchScenes:
         if upload:
             self.upload()
         lib = _lib.load()
-        _lib.check(lib.ehss_scenes_build_ex(len(self.scenes), self._xyz_ptrs, self._r_ptrs, self._n, self.leaf_size,
-                                            self._scenes, self._sizes, self.ws_ptr, self.ws_bytes, self.flags,
-                                            stream_handle(self.device)), 'batched scene build')
+        _lib.check(lib.ehss_scenes_build_centred(len(self.scenes), self._xyz_ptrs, self._r_ptrs, self._n, self.leaf_size,
+                                                 self._scenes, self._sizes, self.ws_ptr, self.ws_bytes, self.flags,
+                                                 self._centers.ctypes.data, stream_handle(self.device)),
+                   'batched scene build')
 
     def drop_build_buffers(self):
         """Free the builder's workspace and the device coordinates once the
@@ -137,21 +131,30 @@ class BatchScenes:
         pinned staging buffers; returns their enclosing radii."""
         if len(structures) != len(self.scenes):
             raise ValueError('Refit requires fixed primitive identities.')
-        hx, hr = self.h_xyz.numpy(), self.h_r.numpy()
-        radii = []
-        for (c, r), a0, n in zip(structures, self.atom0, self.n_atoms):
-            c = np.ascontiguousarray(c, dtype=np.float64); r = np.ascontiguousarray(r, dtype=np.float64)
-            if c.shape != (n, 3) or r.shape != (n,):
-                raise ValueError('Refit requires fixed primitive identities.')
-            if not np.isfinite(c).all() or not np.isfinite(r).all() or np.any(r <= 0):
-                raise ValueError('Finite centers (N,3) and positive finite radii required.')
-            radii.append(enclosing_radius(c, r))
         # an earlier upload from the staging buffers may still be in flight
         torch().cuda.current_stream(self.device).synchronize()
-        for (c, r), a0, n in zip(structures, self.atom0, self.n_atoms):
-            hx[3 * a0:3 * (a0 + n)] = np.asarray(c, dtype=np.float64).ravel()
-            hr[a0:a0 + n] = r
-        return radii
+        return self._stage(structures, 'Refit requires fixed primitive identities.')
+
+    def _stage(self, structures, shape_error):
+        """Checks and copies every structure into the pinned buffers
+        (ehss_stage_structures); keeps the centres, returns the radii."""
+        S = len(structures)
+        keep, xyz, r = [], [], []
+        for (c, q), n in zip(structures, self.n_atoms.tolist()):
+            c, q = np.ascontiguousarray(c, dtype=np.float64), np.ascontiguousarray(q, dtype=np.float64)
+            if c.shape != (n, 3) or q.shape != (n,):
+                raise ValueError(shape_error)
+            keep.append((c, q))
+            xyz.append(c.__array_interface__['data'][0])
+            r.append(q.__array_interface__['data'][0])
+        centers, radii = np.empty((S, 3)), np.empty(S)
+        rc = _lib.load().ehss_stage_structures(S, (ct.c_void_p * S)(*xyz), (ct.c_void_p * S)(*r), self.n_atoms.ctypes.data,
+                                               self.h_xyz.data_ptr(), self.h_r.data_ptr(), centers.ctypes.data,
+                                               radii.ctypes.data)
+        if rc:
+            raise ValueError('Finite centers (N,3) and positive finite radii required.')
+        self._centers = centers
+        return radii.tolist()
 
     def refit(self, structures):
         """New coordinates of the same structures with every tree's topology

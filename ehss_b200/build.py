@@ -18,7 +18,8 @@ HERE = Path(__file__).resolve().parent
 CSRC = HERE / 'csrc'
 ROOT = HERE.parent
 LIB = HERE / 'libehss_b200.so'
-SOURCES = ['capi.cu', 'scene.cu', 'trace.cu', 'pa_grid.cu', 'compact.cu', 'noalloc.cu', 'sobol_host.cpp']
+SOURCES = ['capi.cu', 'scene.cu', 'trace.cu', 'pa_grid.cu', 'compact.cu', 'noalloc.cu', 'sobol_host.cpp',
+           'stage_host.cpp']
 HEADERS = ['ehss_internal.cuh']
 ARCH = ['-gencode', 'arch=compute_100a,code=sm_100a']
 
@@ -42,7 +43,7 @@ def build(force=False, verbose=False, ptxas_verbose=False):
     if not force and not stale():
         return LIB
     tmp = LIB.with_suffix('.so.tmp')
-    cmd = [nvcc(), *ARCH, '-O3', '-lineinfo', '-std=c++17', '--shared', '-Xcompiler', '-fPIC',
+    cmd = [nvcc(), *ARCH, '-O3', '-lineinfo', '-std=c++17', '--shared', '-Xcompiler', '-fPIC,-ffp-contract=off',
            '-I', str(ROOT / 'include'), '-o', str(tmp), *[str(CSRC / s) for s in SOURCES], '-cudart', 'static']
     if ptxas_verbose:
         cmd[1:1] = ['-Xptxas', '-v']

@@ -112,26 +112,8 @@ int ehss_compact_source_rays(const ehss_boundary* boundary_host, int log2n, uint
 int ehss_enclosing_radius(int64_t n_atoms, const double* xyz, const double* radii, double* radius) {
     clear_error();
     if (n_atoms < 1 || !xyz || !radii || !radius) { set_error("invalid arguments"); return EHSS_ERR_VALUE; }
-    // k_stats' operations: sequential column sums divided by n, then max of |c - centre| + r
-    // (norm as sqrt((x*x + y*y) + z*z)), times 1.000000001; each operation rounded once
-    volatile double acc[3] = {0., 0., 0.};
-    for (int64_t i = 0; i < n_atoms; ++i)
-        for (int c = 0; c < 3; ++c) acc[c] = acc[c] + xyz[3 * i + c];
     double center[3];
-    for (int c = 0; c < 3; ++c) center[c] = acc[c] / (double)n_atoms;
-    double smax = 0.;
-    bool nan = false;
-    for (int64_t i = 0; i < n_atoms; ++i) {
-        volatile double x = xyz[3 * i] - center[0], y = xyz[3 * i + 1] - center[1], z = xyz[3 * i + 2] - center[2];
-        volatile double xx = x * x, yy = y * y, zz = z * z;
-        volatile double s = xx + yy;
-        s = s + zz;
-        volatile double len = std::sqrt((double)s);
-        len = len + radii[i];
-        if (std::isnan((double)len)) nan = true;
-        else if (len > smax) smax = len;
-    }
-    *radius = nan ? NAN : smax * 1.000000001;
+    enclosing_sphere(n_atoms, xyz, radii, center, radius);
     return EHSS_OK;
 }
 
@@ -196,6 +178,21 @@ int ehss_scenes_build_ex(int n_scenes, const double* const* xyz_dev, const doubl
     if (flags & ~EHSS_BUILD_EXTERIOR) { set_error("unknown build flags 0x%x", flags); return EHSS_ERR_VALUE; }
     return build_scenes(n_scenes, xyz_dev, radii_dev, n_atoms_host, leaf_size, scenes_dev, scene_bytes_host,
                         workspace_dev, workspace_bytes, as_stream(stream), (flags & EHSS_BUILD_EXTERIOR) != 0);
+}
+
+int ehss_scenes_build_centred(int n_scenes, const double* const* xyz_dev, const double* const* radii_dev,
+                              const int64_t* n_atoms_host, int leaf_size, void* const* scenes_dev,
+                              const uint64_t* scene_bytes_host, void* workspace_dev, uint64_t workspace_bytes,
+                              uint32_t flags, const double* centers_host, void* stream) {
+    clear_error();
+    if (n_scenes < 1 || !xyz_dev || !radii_dev || !n_atoms_host || !scenes_dev || !scene_bytes_host ||
+        !workspace_dev || !centers_host) {
+        set_error("invalid arguments");
+        return EHSS_ERR_VALUE;
+    }
+    if (flags & ~EHSS_BUILD_EXTERIOR) { set_error("unknown build flags 0x%x", flags); return EHSS_ERR_VALUE; }
+    return build_scenes(n_scenes, xyz_dev, radii_dev, n_atoms_host, leaf_size, scenes_dev, scene_bytes_host,
+                        workspace_dev, workspace_bytes, as_stream(stream), (flags & EHSS_BUILD_EXTERIOR) != 0, centers_host);
 }
 
 int ehss_scenes_refit(int n_scenes, const double* const* xyz_dev, const double* const* radii_dev,
@@ -405,6 +402,11 @@ int ehss_blocks_prepare(ehss_block* blocks, int n_blocks, const uint64_t* seeds,
         return EHSS_ERR_VALUE;
     }
     int64_t total = 0, hist = 0;
+    // blocks of one call that share seed and ray count share the enumeration (the frames of an ensemble do):
+    // made once, about 10 us each, and copied.  kSeen: the last block of each hash.
+    constexpr int kSeen = 256;
+    int seen[kSeen];
+    for (int& s : seen) s = -1;
     for (int b = 0; b < n_blocks; ++b) {
         ehss_block& B = blocks[b];
         if (!B.scene) { set_error("block %d: null scene", b); return EHSS_ERR_VALUE; }
@@ -417,11 +419,18 @@ int ehss_blocks_prepare(ehss_block* blocks, int n_blocks, const uint64_t* seeds,
         if (!(B.flags & (EHSS_BLOCK_EHSS | EHSS_BLOCK_PA))) { set_error("block %d: no work flags", b); return EHSS_ERR_VALUE; }
         if (B.hist_offset < 0) B.hist_offset = hist;
         hist = B.hist_offset + B.cap + 1;
-        uint32_t sv[4 * 30], shift[4];
-        sobol_scramble(4, seeds[b], sv, shift);
-        if (!sobol_coherent_order(B.log2_rays, sv, shift, &B.basis[0][0], B.base)) {
-            set_error("block %d: no coherent enumeration", b);
-            return EHSS_ERR_VALUE;
+        int& like = seen[((seeds[b] ^ (seeds[b] >> 32)) * 31 + (uint64_t)B.log2_rays) % kSeen];
+        if (like >= 0 && seeds[like] == seeds[b] && blocks[like].log2_rays == B.log2_rays) {
+            std::memcpy(B.basis, blocks[like].basis, sizeof(B.basis));
+            std::memcpy(B.base, blocks[like].base, sizeof(B.base));
+        } else {
+            uint32_t sv[4 * 30], shift[4];
+            sobol_scramble(4, seeds[b], sv, shift);
+            if (!sobol_coherent_order(B.log2_rays, sv, shift, &B.basis[0][0], B.base)) {
+                set_error("block %d: no coherent enumeration", b);
+                return EHSS_ERR_VALUE;
+            }
+            like = b;
         }
         if (B.flags & EHSS_BLOCK_RAYS) {
             if (!B.rays || !(B.ray_scale > 0.) || !std::isfinite(B.ray_scale)) {

@@ -230,6 +230,7 @@ bool sobol_scramble(int dim, uint64_t seed, uint32_t* sv, uint32_t* shift);
 bool sobol_coherent_order(int m, const uint32_t* sv, const uint32_t* shift, uint32_t* basis, uint32_t* base);
 void sobol_direction_numbers(int dim, uint32_t* v);
 int sm_count();
+void enclosing_sphere(int64_t n, const double* xyz, const double* radii, double* center, double* radius);
 void sobol4_params(uint64_t seed, Sobol4Params* p);
 uint64_t build_workspace_bytes(int64_t N, int S);
 int build_scenes(int S, const double* const* xyz, const double* const* radii, const int64_t* n, int leaf_size,

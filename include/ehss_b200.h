@@ -147,6 +147,25 @@ int ehss_scenes_build_ex(int n_scenes, const double* const* xyz_dev, const doubl
                          const uint64_t* scene_bytes_host, void* workspace_dev, uint64_t workspace_bytes,
                          uint32_t flags, void* stream);
 
+/* ehss_scenes_build_ex with the structures' centres given: centers_host[3 n]
+ * holds each one's mean, summed in row order as ehss_stage_structures does (the
+ * device's own chain of that many dependent additions is most of a small
+ * build's statistics).  Everything else is computed from the coordinates. */
+int ehss_scenes_build_centred(int n_scenes, const double* const* xyz_dev, const double* const* radii_dev,
+                              const int64_t* n_atoms_host, int leaf_size, void* const* scenes_dev,
+                              const uint64_t* scene_bytes_host, void* workspace_dev, uint64_t workspace_bytes,
+                              uint32_t flags, const double* centers_host, void* stream);
+
+/* Host arrays of many structures into one staging buffer each: checks that
+ * every coordinate is finite and every radius positive and finite
+ * (EHSS_ERR_VALUE, nothing written to the staging buffers, otherwise), copies
+ * structure after structure into xyz_out and radii_out, and writes each one's
+ * centre (centers_out[3 n]) and impact-disk radius (enclosing_out[n], as
+ * ehss_enclosing_radius).  Host only. */
+int ehss_stage_structures(int n_structures, const double* const* xyz_host, const double* const* radii_host,
+                          const int64_t* n_atoms, double* xyz_out, double* radii_out, double* centers_out,
+                          double* enclosing_out);
+
 /* Refit: new coordinates (and radii) for scenes built without
  * EHSS_BUILD_EXTERIOR, same atom count and identities, tree topology kept.
  * Replaces SphereIndex.refit (pa_spatial.py:166-170, which raises
