@@ -14,8 +14,8 @@ namespace ehss {
 //
 //   SceneHeader                              256 B
 //   nodes   float4[8 * n_nodes]              4-wide nodes (below), child boxes in FP32
-//   atoms   float4[n]      (x, y, z, r)      FP32, centre relative to header.center,
-//                                            in leaf order
+//   atoms   float4[n]      (x, y, z, k)      FP32, centre c relative to header.center,
+//                                            k = (r^2 - |c|^2) / 2, in leaf order
 //   atoms64 double4[n]     (x, y, z, r)      FP64 reference values, leaf order
 //   ids     int32[n]       leaf order -> input atom id
 //   rank    int32[n]       input atom id -> leaf order

@@ -161,9 +161,9 @@ __device__ __noinline__ void row_span(double cx, double cy, double r, double low
 // |k - (x0 + fx)| <= sqrt(r^2 - (y - y0 - fy)^2).
 //
 // Error bounds of the FP32 row ends (u = 2^-24, r the radius in pixels).
-// The radius is the scene's FP32 one.  fx, fy and r2 are rounded once from FP64, y - y0 is an exact integer below
+// fx, fy and r2 are rounded once from FP64, y - y0 is an exact integer below
 // r + 2 in magnitude and dy = (y - y0) - fy is off by at most u (r + 1), so
-// rem = r2 - dy^2 is off by at most u (6 r^2 + 3 r + 1); tol is u (8 r^2 + 6 r + 4).
+// rem = r2 - dy^2 is off by at most u (4 r^2 + 3 r + 1); tol is u (8 r^2 + 6 r + 4).
 // rem >= 4 tol bounds the error of sqrt(rem) by tol / sqrt(rem); rsqrtf's
 // 2 ulp, the product and fx -/+ half add less than 2^-21 (half + 1), of which
 // the bound takes twice.  FP64's own roundings are below 1e-9 pixel.
@@ -299,18 +299,18 @@ __global__ void __launch_bounds__(512) k_grid_cover(const void* scene, int m_max
         const int end = min(places, begin + size), cnt = 8 * (end - begin);
         for (int k0 = threadIdx.x; k0 < ((cnt + 31) & ~31); k0 += kStageLoads * blockDim.x) {
             double2 c[kStageLoads];
-            float r[kStageLoads];
+            double r[kStageLoads];
             int j[kStageLoads];
 #pragma unroll
             for (int i = 0; i < kStageLoads; ++i) {
                 const int k = k0 + i * (int)blockDim.x;
                 j[i] = k < cnt ? 8 * spread_run(begin + (k >> 3), bits, width) + (k & 7) : m;
                 c[i] = xy[min(j[i], m - 1)];
-                r[i] = S.atoms[min(j[i], m - 1)].w;
+                r[i] = S.atoms64[min(j[i], m - 1)].w;
             }
 #pragma unroll
             for (int i = 0; i < kStageLoads; ++i) {
-                const double cx = (c[i].x - lower) * inv - .5, cy = (c[i].y - lower) * inv - .5, rp = (double)r[i] * inv;
+                const double cx = (c[i].x - lower) * inv - .5, cy = (c[i].y - lower) * inv - .5, rp = r[i] * inv;
                 const double flx = floor(cx), fly = floor(cy);
                 const float4 d = make_float4((float)(cx - flx), (float)(cy - fly), (float)(rp * rp), (float)rp);
                 const int2 o = make_int2((int)flx, (int)fly);

@@ -513,6 +513,12 @@ __global__ void k_refit(const BuildDesc* descs, const int32_t* atom_scene, int64
     }
 }
 
+// FP32 atom record (see ehss_internal.cuh) of a centre relative to the scene's.
+__device__ __forceinline__ float4 atom_record(double x, double y, double z, double r) {
+    return make_float4(__double2float_rn(x), __double2float_rn(y), __double2float_rn(z),
+                       __double2float_rn(0.5 * (r * r - (x * x + y * y + z * z))));
+}
+
 // 4-wide node record i (see ehss_internal.cuh) from up to four child slots.
 __device__ __forceinline__ void write_node4(float4* nodes, int64_t i, const float (*box)[6], const int* ref, int n,
                                             float eps) {
@@ -609,8 +615,7 @@ __device__ __forceinline__ void emit_atom(const BuildDesc& D, const SceneHeader*
     int32_t* ids = reinterpret_cast<int32_t*>(D.scene + H->off_ids);
     int32_t* rank = reinterpret_cast<int32_t*>(D.scene + H->off_rank);
     double x = D.xyz[a * 3], y = D.xyz[a * 3 + 1], z = D.xyz[a * 3 + 2], r = D.radii[a];
-    atoms[j] = make_float4(__double2float_rn(x - H->center[0]), __double2float_rn(y - H->center[1]),
-                           __double2float_rn(z - H->center[2]), __double2float_rn(r));
+    atoms[j] = atom_record(x - H->center[0], y - H->center[1], z - H->center[2], r);
     atoms64[j] = make_double4(x, y, z, r);
     ids[j] = (int32_t)a;
     rank[a] = (int32_t)j;
@@ -844,8 +849,7 @@ __global__ void k_refit_atoms(const BuildDesc* descs, const int32_t* atom_scene,
     float4* atoms = reinterpret_cast<float4*>(D.scene + H->off_atoms);
     double4* atoms64 = reinterpret_cast<double4*>(D.scene + H->off_atoms64);
     double x = D.xyz[a * 3], y = D.xyz[a * 3 + 1], z = D.xyz[a * 3 + 2], r = D.radii[a];
-    atoms[j] = make_float4(__double2float_rn(x - H->center[0]), __double2float_rn(y - H->center[1]),
-                           __double2float_rn(z - H->center[2]), __double2float_rn(r));
+    atoms[j] = atom_record(x - H->center[0], y - H->center[1], z - H->center[2], r);
     atoms64[j] = make_double4(x, y, z, r);
     float b[6];
     atom_box(D.xyz, D.radii, H->center, a, b);
@@ -1046,7 +1050,8 @@ __global__ void __launch_bounds__(32 * kExposureWarps, 4) k_exposure(BuildDesc* 
         BuildDesc& D = descs[atom_scene[g]];
         const SceneView S = scene_view(D.scene);
         const int j = (int)(g - D.atom0);          // leaf-order position: neighbouring warps share subtrees
-        const float4 b = S.atoms[j];
+        float4 b = S.atoms[j];
+        b.w = __double2float_rn(S.atoms64[j].w);       // radius
         const float mS = 2e-6f * S.h->scale_f;
         const float h_fine = b.w * rho_c;
         if (lane == 0) {
@@ -1118,7 +1123,8 @@ __global__ void __launch_bounds__(32 * kExposureWarps, 4) k_exposure(BuildDesc* 
             }
             const int k = ((~W.leaves[lo_l]) >> kLeafBits) + t - (lo_l ? leaf_end[lo_l - 1] : 0);
             if (k >= S.h->n_atoms || k == j) continue;
-            const float4 a = S.atoms[k];
+            float4 a = S.atoms[k];
+            a.w = __double2float_rn(S.atoms64[k].w);   // radius
             const float dx = a.x - b.x, dy = a.y - b.y, dz = a.z - b.z;
             const float d = sqrtf(dx * dx + dy * dy + dz * dz);
             if (d + b.w <= a.w - 1e-4f * (b.w + d + a.w) - mS) { W.whole = 1; continue; }   // C alone holds B

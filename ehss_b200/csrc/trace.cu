@@ -17,10 +17,9 @@
 //   EXACT (EHSS_PREC_FP64): every reached sphere is tested in FP64, with the
 //     reference's formula unless an FP64 discriminant shows a certain miss;
 //     U is the running best distance rounded up.
-//   FILTER (EHSS_PREC_FP32): spheres are tested in FP32 with the
-//     cancellation-free perpendicular-distance discriminant
-//     disc = r^2 - |v - (v.d) d|^2 (the fused kernel: the shorter
-//     b^2 + (r^2 - |v|^2) under a widened bound) and a per-ray error bound
+//   FILTER (EHSS_PREC_FP32): spheres are tested in FP32 with a discriminant
+//     formed from the ray's point nearest the structure's centre (seven
+//     operations a sphere, sphere_disc below) and error bounds
 //     (Ep on projections, Edisc on the discriminant).  Certain misses are dropped;
 //     certain hits give an interval [t - Et, t + Et] and lower U to t + Et;
 //     every sphere whose lower bound is <= U (certain or near-tangent) is
@@ -50,9 +49,17 @@ struct LocalStats {
     __device__ LocalStats() : box(0), sphere(0), queries(0), grazing(0), fallback(0), fp64(0), errors(0) {}
 };
 
+// FP32 copy of a ray in the scene frame (centre at the origin): the line's point
+// o nearest the centre, d / sqrt 2, the inverse direction, and the two
+// thresholds of the sphere test.  With x(tau) = o + tau d the ray starts at
+// tau0, and t = tau - tau0.
+//   thr  = (|o|^2 - Edisc) / 2
+//   bmin = (tau0 - Ep) / sqrt 2
 struct RayF {
-    float ox, oy, oz, dx, dy, dz, ix, iy, iz, Ep, Edisc;
+    float ox, oy, oz, dx, dy, dz, ix, iy, iz, thr, bmin;
 };
+
+constexpr float kSqrt2 = 1.41421356f, kHalfSqrt2 = 0.707106781f;
 
 // Inverse direction component for the box tests, from the fast quotient
 // (within 2 ulp for these arguments, whose magnitude lies in [1e-20, 1]).  A
@@ -60,71 +67,76 @@ struct RayF {
 // t below 6 S (origins within 3 S, boxes within S) that is under 1.5e-6 S
 // even with the slab's own roundings, well inside the 2^-14 S (6.1e-5 S) by
 // which every node box is widened, and the sign, which picks the near plane,
-// is exact.
+// is exact.  The start's distance along the line enters a crossing with d inv in
+// place of 1 (3u |tau0|) and less Ep: another 3.5e-6 S.
 __device__ __forceinline__ float safe_rcp(float x) {
     float a = fabsf(x) < 1e-20f ? copysignf(1e-20f, x) : x;
     return __fdividef(1.0f, a);
 }
 
-// FP32 copy of an FP64 ray in the scene frame; false when the origin is too
-// far from the centre for the FP32 error bounds (or not finite).  widen > 0
-// adds widen * (rmax^2 + A^2) to the discriminant bound, for the fused
-// kernel's shorter discriminant (kWidenShortDisc below).
-__device__ __forceinline__ bool setup_ray(const SceneHeader* H, const double* o, const double* d, RayF& r,
-                                          float widen = 0.0f) {
-    r.ox = __double2float_rn(o[0] - H->center[0]);
-    r.oy = __double2float_rn(o[1] - H->center[1]);
-    r.oz = __double2float_rn(o[2] - H->center[2]);
-    r.dx = __double2float_rn(d[0]); r.dy = __double2float_rn(d[1]); r.dz = __double2float_rn(d[2]);
-    float S = H->scale_f;
-    float a = sqrtf(fmaf(r.ox, r.ox, fmaf(r.oy, r.oy, r.oz * r.oz)));
-    if (!(a <= 3.0f * S)) return false;
-    r.ix = safe_rcp(r.dx); r.iy = safe_rcp(r.dy); r.iz = safe_rcp(r.dz);
-    float A = a + S;
-    r.Ep = A * (32.0f * kU32);
-    float rm = H->rmax_f;
-    r.Edisc = (8.0f * kU32) * rm * rm + 2.5f * rm * r.Ep + 8.0f * r.Ep * r.Ep;
-    if (widen > 0.0f) r.Edisc += widen * (rm * rm + A * A);
-    return true;
-}
+// Error bounds of the FP32 sphere test, from the scene's scale S alone
+// (|c| + r <= S for every atom; |o| <= S (1 + 1e-5), since a line farther out
+// meets none; u = 2^-24).  In exact arithmetic, with o.d = 0 and |d| = 1,
+//     disc = r^2 - |c - o|^2 + (c.d)^2 = 2 (D - |o|^2 / 2),
+//     D = (c.d / sqrt 2)^2 + c.o + k,   k = (r^2 - |c|^2) / 2 per atom.
+// 2 D is off by at most: k rounded once, u S^2; c and o rounded, 2u S |o| each;
+// b = c.d / sqrt 2 from rounded c and d (twice) and three roundings, 6u S, so
+// 12u S^2 on its square; the three sums of c.o + k, 3u (S^2 + 2 S |o|); the last
+// fma, 2u S (S + |o|); the threshold's own rounding, 2u |o|^2: together at most
+// 18u S^2 + 12u S |o| + 2u |o|^2 <= 33u S^2.  Edisc = 48u S^2.
+// t-units: b sqrt 2 - tau0 is off by 9u S from b, and |tau0|, |t| <= 4 S round
+// by u each at most three times: 21u S.  Ep = 48u S.
+constexpr float kEdisc = 48.0f * kU32, kEp = 48.0f * kU32;
 
-// setup_ray for the EXACT walk.  Its FP64 reject takes |d| = 1; a direction off by more than 1e-11 in |d|^2 (which
-// moves disc by 1e-11 A^2, below the bounds for A < 10^6 rmax) switches it off with infinite bounds.
-__device__ __forceinline__ bool setup_exact(const SceneHeader* H, const double* o, const double* d, RayF& r) {
-    if (!setup_ray(H, o, d, r)) return false;
+__device__ __forceinline__ float ray_edisc(const SceneHeader* H) { const float S = __ldg(&H->scale_f); return kEdisc * S * S; }
+__device__ __forceinline__ float ray_ep(const SceneHeader* H) { return kEp * __ldg(&H->scale_f); }
+
+constexpr int kRayFar = 0, kRayOk = 1, kRayNotUnit = 2;
+
+// FP32 copy of an FP64 ray.  kRayFar: the origin is beyond 3 S from the centre
+// (or not finite), where node boxes are not widened enough.  kRayNotUnit: the
+// direction is off by more than 1e-11 in |d|^2, which the sphere test's
+// identity does not allow (boxes still hold: o is then the ray's own origin).
+__device__ __forceinline__ int setup_ray(const SceneHeader* H, const double* o, const double* d, RayF& r) {
+    const double x = o[0] - H->center[0], y = o[1] - H->center[1], z = o[2] - H->center[2];
+    const float S = H->scale_f;
+    const float fx = (float)x, fy = (float)y, fz = (float)z;
+    if (!(sqrtf(fmaf(fx, fx, fmaf(fy, fy, fz * fz))) <= 3.0f * S)) return kRayFar;
     const double aa = fma(d[0], d[0], fma(d[1], d[1], d[2] * d[2]));
-    if (!(fabs(aa - 1.0) <= 1e-11)) r.Ep = r.Edisc = CUDART_INF_F;
-    return true;
+    const bool unit = fabs(aa - 1.0) <= 1e-11;
+    const double tau0 = unit ? fma(x, d[0], fma(y, d[1], z * d[2])) : 0.0;
+    r.ox = (float)fma(-tau0, d[0], x);
+    r.oy = (float)fma(-tau0, d[1], y);
+    r.oz = (float)fma(-tau0, d[2], z);
+    const float dx = (float)d[0], dy = (float)d[1], dz = (float)d[2];
+    r.ix = safe_rcp(dx); r.iy = safe_rcp(dy); r.iz = safe_rcp(dz);
+    r.dx = dx * kHalfSqrt2; r.dy = dy * kHalfSqrt2; r.dz = dz * kHalfSqrt2;
+    const float q = fmaf(r.ox, r.ox, fmaf(r.oy, r.oy, r.oz * r.oz));
+    // a line beyond S passes every sphere by 1e-5 S: all tests miss
+    r.thr = q > 1.00002f * S * S ? CUDART_INF_F : 0.5f * (q - kEdisc * S * S);
+    r.bmin = ((float)tau0 - kEp * S) * kHalfSqrt2;
+    return unit ? kRayOk : kRayNotUnit;
 }
 
-// The fused kernel's FILTER leaf test forms disc = b^2 + (r^2 - |v|^2)
-// (two operations fewer, and a dependency chain three shorter, than
-// r^2 - |v - b d|^2; v = c - o, b = v.d, both computed as in the
-// cancellation-free form).  In exact arithmetic on the FP32 values the two
-// differ by 2 b db + b^2 (|d|^2 - 1), db the rounding of b (<= 3u |v|) and
-// | |d|^2 - 1 | <= 2.1u: at most 8.2u |v|^2.  Rounding r^2 - |v|^2 costs at
-// most 4u (|v|^2 + r^2) and the last fma u |disc|; the cancellation-free
-// value's own roundings, already inside Edisc, are at most 5.1u |v - b d|^2 +
-// u |disc| again, and where a classification depends on them (true disc >= 0,
-// or computed disc >= 2 Edisc) |v - b d|^2 <= rmax^2 + 2 Edisc.  With
-// |v| <= |o| + S <= A (1 + 4u) the difference stays below 12.3u A^2 + 11.1u
-// rmax^2, so adding 16u (rmax^2 + A^2) to Edisc keeps every certain miss,
-// certain-hit interval and grazing lower bound as sound as before (u = 2^-24).
-constexpr float kWidenShortDisc = 16.0f * kU32;
+// D (above) of atom a = (c, k) and b = c.d / sqrt 2.
+__device__ __forceinline__ float sphere_disc(const RayF& r, const float4& a, float& b) {
+    b = fmaf(a.x, r.dx, fmaf(a.y, r.dy, a.z * r.dz));
+    return fmaf(b, b, fmaf(a.x, r.ox, fmaf(a.y, r.oy, fmaf(a.z, r.oz, a.w))));
+}
 
 // sqrt(disc) of a certain hit (computed disc >= 2 Edisc) and the error bound Et
-// of its entry and exit distances b -/+ sqrt(disc), from one reciprocal square
+// of its entry and exit distances bt -/+ sqrt(disc), from one reciprocal square
 // root: s = disc * y and Edisc / s = Edisc * y.  rsqrtf is within 2 ulp of 1/sqrt(disc) (the CUDA
 // math library's stated bound; at most 2.09 u measured over every float in
 // [2^-14, 2^8)), so s is within 5.01 u of sqrt(disc) and Edisc * y within
-// 5.01 u of Edisc / sqrt(disc).  With the roundings of s and of b -/+ s the
-// distance error stays below Ep + Edisc / sqrt(disc) + 6.01 u (|b| + s), which Et
-// covers with a factor-2 margin on its first two terms, as the correctly
-// rounded square root and quotient did before (u = 2^-24).
-__device__ __forceinline__ float certain_sqrt(float b, float disc, const RayF& r, float& Et) {
+// 5.01 u of Edisc / sqrt(disc).  With the roundings of disc from D (2u), of s
+// and of bt -/+ s the distance error stays below Ep + Edisc / sqrt(disc) +
+// 8.1 u (|bt| + s), which Et covers with a factor-2 margin on its first two
+// terms.
+__device__ __forceinline__ float certain_sqrt(float bt, float disc, float Ep, float Edisc, float& Et) {
     const float y = rsqrtf(disc);
     const float s = disc * y;
-    Et = 2.0f * (r.Ep + r.Edisc * y) + 8.0f * kU32 * (fabsf(b) + s);
+    Et = 2.0f * (Ep + Edisc * y) + 12.0f * kU32 * (fabsf(bt) + s);
     return s;
 }
 
@@ -145,9 +157,9 @@ __device__ __forceinline__ float min3f(float a, float b, float c) {
 // rounding is monotone, so the near plane's distance is the slab minimum the
 // textbook test forms with fminf, bit for bit.  An unused slot holds the box
 // lo = +inf, hi = -inf, whose near distance is +inf on every axis, so it
-// misses without a check of its reference.  oi = o * inv per axis, formed
-// once per node visit (held per lane it would cost three registers of the
-// fused kernel).
+// misses without a check of its reference.  oi = o * inv + tau0 per axis
+// (distances from the ray's start), formed once per node visit (held per lane
+// it would cost three registers of the fused kernel).
 __device__ __forceinline__ float box_enter(const RayF& r, float oix, float oiy, float oiz, float nx, float fx, float ny,
                                            float fy, float nz, float fz, float U) {
     float tnx = fmaf(nx, r.ix, -oix), tfx = fmaf(fx, r.ix, -oix);
@@ -182,7 +194,9 @@ __device__ __forceinline__ Hits4 visit4(const float4* nodes, int node, const Ray
     Hits4 h;
     h.ref[0] = __float_as_int(rf.x); h.ref[1] = __float_as_int(rf.y);
     h.ref[2] = __float_as_int(rf.z); h.ref[3] = __float_as_int(rf.w);
-    const float oix = r.ox * r.ix, oiy = r.oy * r.iy, oiz = r.oz * r.iz;
+    // distances from the ray's start (less Ep, which the boxes' widening absorbs)
+    const float tau0 = r.bmin * kSqrt2;
+    const float oix = fmaf(r.ox, r.ix, tau0), oiy = fmaf(r.oy, r.iy, tau0), oiz = fmaf(r.oz, r.iz, tau0);
     h.t[0] = box_enter(r, oix, oiy, oiz, nx.x, fx.x, ny.x, fy.x, nz.x, fz.x, U);
     h.t[1] = box_enter(r, oix, oiy, oiz, nx.y, fx.y, ny.y, fy.y, nz.y, fz.y, U);
     h.t[2] = box_enter(r, oix, oiy, oiz, nx.z, fx.z, ny.z, fy.z, nz.z, fz.z, U);
@@ -199,7 +213,7 @@ __device__ __forceinline__ bool better(double dist, int id, double best, int bes
 }
 
 // FP64 all-atom nearest search (origins far from the structure).
-__device__ __noinline__ int nearest_flat(const SceneView& S, const double* o, const double* d, int last_rank, double& best_out,
+__device__ __forceinline__ int nearest_flat(const SceneView& S, const double* o, const double* d, int last_rank, double& best_out,
                             LocalStats& st) {
     int n = S.h->n_atoms;
     double best = CUDART_INF;
@@ -217,17 +231,17 @@ __device__ __noinline__ int nearest_flat(const SceneView& S, const double* o, co
 }
 
 // Nearest entry: returns the leaf-order rank of the collider (or -1) and its
-// FP64 entry distance, identical to the reference's choice.  The explicit-ray
-// kernels and the fused kernel's overflow fallback use it; it restates the
-// Walker's FP32 filter in a self-contained form because the fused kernel's
-// local-memory frame includes this function's, and a Walker-based version
-// (with a LaneRay copy) measured 0.9 % slower on the batched trace.
+// FP64 entry distance, identical to the reference's choice.  Parked rays
+// (rest_of_path, EXACT) and the cap extension use it.
 template <bool EXACT>
-__device__ __noinline__ int nearest(const SceneView& S, const double* o, const double* d, int last_rank,
+__device__ __forceinline__ int nearest(const SceneView& S, const double* o, const double* d, int last_rank,
                                     double& best_out, LocalStats& st) {
     ++st.queries;
     RayF r;
-    if (!setup_ray(S.h, o, d, r)) return nearest_flat(S, o, d, last_rank, best_out, st);
+    const int kind = setup_ray(S.h, o, d, r);
+    if (kind == kRayFar) return nearest_flat(S, o, d, last_rank, best_out, st);
+    if (!EXACT && kind == kRayNotUnit) { --st.queries; return nearest<true>(S, o, d, last_rank, best_out, st); }
+    const float Edisc = ray_edisc(S.h), Ep = ray_ep(S.h);
     float U = CUDART_INF_F;
     double best = CUDART_INF;
     int best_rank = -1, best_id = -1;
@@ -273,18 +287,16 @@ __device__ __noinline__ int nearest(const SceneView& S, const double* o, const d
                         U = __double2float_ru(best);
                     }
                 } else {
-                    float4 a = __ldg(S.atoms + k);
-                    float vx = a.x - r.ox, vy = a.y - r.oy, vz = a.z - r.oz;
-                    float b = fmaf(vx, r.dx, fmaf(vy, r.dy, vz * r.dz));
-                    float px = fmaf(-b, r.dx, vx), py = fmaf(-b, r.dy, vy), pz = fmaf(-b, r.dz, vz);
-                    float q = fmaf(px, px, fmaf(py, py, pz * pz));
-                    float disc = fmaf(a.w, a.w, -q);
-                    if (disc < -r.Edisc || b < -r.Ep) continue;          // certain miss
+                    const float4 a = __ldg(S.atoms + k);
+                    float b;
+                    const float D = sphere_disc(r, a, b);
+                    if (D < r.thr || b < r.bmin) continue;               // certain miss
+                    const float disc = fmaf(2.0f, D - r.thr, -Edisc), bt = fmaf(b - r.bmin, kSqrt2, -Ep);
                     float lo;
                     bool certain = false;
-                    if (disc >= 2.0f * r.Edisc) {
+                    if (disc >= 2.0f * Edisc) {
                         float Et;
-                        const float t = b - certain_sqrt(b, disc, r, Et);
+                        const float t = bt - certain_sqrt(bt, disc, Ep, Edisc, Et);
                         if (t < -2.0f * Et) continue;                    // origin inside: no entry ahead
                         if (t > Et) {
                             certain = true;
@@ -294,7 +306,7 @@ __device__ __noinline__ int nearest(const SceneView& S, const double* o, const d
                         }
                     }
                     if (!certain) {
-                        lo = fmaxf(0.0f, (b - r.Ep - sqrtf(fmaxf(disc, 0.0f) + r.Edisc)) * (1.0f - 8.0f * kU32));
+                        lo = fmaxf(0.0f, (bt - Ep - sqrtf(fmaxf(disc, 0.0f) + Edisc)) * (1.0f - 8.0f * kU32));
                         grazing = true;
                     }
                     if (lo <= U) {
@@ -340,13 +352,20 @@ __device__ __noinline__ int nearest(const SceneView& S, const double* o, const d
     return best_rank;
 }
 
+// The same out of line, for kernels that are not bound by their registers.
+template <bool EXACT>
+__device__ __noinline__ int nearest_call(const SceneView& S, const double* o, const double* d, int last_rank,
+                                         double& best_out, LocalStats& st) {
+    return nearest<EXACT>(S, o, d, last_rank, best_out, st);
+}
+
 // Any-hit PA query (pa_spatial._one with sphere_hit): true when the ray
 // meets any sphere other than owner_rank.
 __device__ __noinline__ bool anyhit(const SceneView& S, const double* o, const double* d, int owner_rank,
                                     LocalStats& st) {
     ++st.queries;
     RayF r;
-    if (!setup_ray(S.h, o, d, r)) {
+    if (setup_ray(S.h, o, d, r) != kRayOk) {
         int n = S.h->n_atoms;
         for (int k = 0; k < n; ++k) {
             if (k == owner_rank) continue;
@@ -356,6 +375,7 @@ __device__ __noinline__ bool anyhit(const SceneView& S, const double* o, const d
         }
         return false;
     }
+    const float Edisc = ray_edisc(S.h), Ep = ray_ep(S.h);
     int stack_ref[kStackDepth];
     int sp = 0;
     int cur = 0;
@@ -380,20 +400,18 @@ __device__ __noinline__ bool anyhit(const SceneView& S, const double* o, const d
             for (int k = first; k < first + cnt; ++k) {
                 if (k == owner_rank) continue;
                 ++st.sphere;
-                float4 a = __ldg(S.atoms + k);
-                float vx = a.x - r.ox, vy = a.y - r.oy, vz = a.z - r.oz;
-                float b = fmaf(vx, r.dx, fmaf(vy, r.dy, vz * r.dz));
-                float px = fmaf(-b, r.dx, vx), py = fmaf(-b, r.dy, vy), pz = fmaf(-b, r.dz, vz);
-                float q = fmaf(px, px, fmaf(py, py, pz * pz));
-                float disc = fmaf(a.w, a.w, -q);
-                if (disc < -r.Edisc) continue;
-                if (disc >= 2.0f * r.Edisc) {
+                const float4 a = __ldg(S.atoms + k);
+                float b;
+                const float D = sphere_disc(r, a, b);
+                if (D < r.thr) continue;
+                const float disc = fmaf(2.0f, D - r.thr, -Edisc), bt = fmaf(b - r.bmin, kSqrt2, -Ep);
+                if (disc >= 2.0f * Edisc) {
                     float Et;
                     // far root: the reference's -b + sqrt(disc) with b = x.d = -(v.d)
-                    const float exitp = b + certain_sqrt(b, disc, r, Et);
+                    const float exitp = bt + certain_sqrt(bt, disc, Ep, Edisc, Et);
                     if (exitp > Et) return true;
                     if (exitp < -2.0f * Et) continue;
-                } else if (b + sqrtf(fmaxf(disc, 0.0f) + r.Edisc) < -2.0f * r.Ep) {
+                } else if (bt + sqrtf(fmaxf(disc, 0.0f) + Edisc) < -2.0f * Ep) {
                     continue;
                 }
                 double4 a64 = S.atoms64[k];
@@ -562,7 +580,7 @@ __device__ __forceinline__ uint4 block_point(const uint4* basis, uint4 base, uin
     return q;
 }
 
-constexpr int kIdle = 0, kTraverse = 1, kDone = 2, kNeedRay = 3;
+constexpr int kIdle = 0, kTraverse = 1, kDone = 2, kNeedRay = 3, kParked = 4;
 // Lanes whose ray has finished wait for a new one until this many of a warp
 // do (16 of 32: the 256-globule batch traces in 23.9 ms against 24.6 with a
 // new ray at once, 24.2 with 8 and 24.2 with 24).
@@ -646,13 +664,17 @@ struct Walker {
         }
         if (leaf != kNoLeaf) {
             leaf_tests(S, leaf, last_rank, L);
-            leaf = kNoLeaf;
-            if (cur < 0) {
-                leaf = cur;
-                cur = pop(sdepth);
-            }
+            next_leaf(sdepth);
         }
     }
+    __device__ __forceinline__ void next_leaf(int sdepth) {
+        leaf = kNoLeaf;
+        if (cur < 0) {
+            leaf = cur;
+            cur = pop(sdepth);
+        }
+    }
+    __device__ __forceinline__ bool finished() const { return cur == kSentinel && leaf == kNoLeaf; }
     __device__ __forceinline__ void add_candidate(int k, float lo) {
         if (lo > U) return;
         bool placed = false;
@@ -668,13 +690,15 @@ struct Walker {
         int first = code >> kLeafBits, cnt = (code & (kMaxLeaf - 1)) + 1;
         if (first + cnt > S.h->n_atoms) { error = true; return; }
         if (COUNT) sphere += cnt - ((unsigned)(last_rank - first) < (unsigned)cnt ? 1 : 0);
-        const double Edisc = EXACT ? (double)r.Edisc : 0., Ep = EXACT ? (double)r.Ep : 0.;
+        // EXACT: the FP64 reject takes |d| = 1 and is off (infinite bounds) for other directions
+        const double slack = EXACT ? (r.thr == CUDART_INF_F ? CUDART_INF : 1.0) : 0.;
+        const double Edisc = EXACT ? ray_edisc(S.h) * slack : 0., Ep = EXACT ? ray_ep(S.h) * slack : 0.;
         for (int k = first; k < first + cnt; ++k) {
             if (EXACT) {
                 // FP64 reject before the reference's formula (two divisions and a square root; 650 atoms,
                 // 20 x 65,536 rays with PA: 1.55 -> 1.09 ms together with PA from the first query):
                 // q = x.d, w = |x|^2 - r^2 and disc = q^2 - w are within 1e-13 A^2 of their true
-                // values for unit d (setup_exact), far inside the FP32 filter's bounds
+                // values for unit d, far inside the FP32 filter's bounds
                 const double4 a = S.atoms64[k];
                 const double x0 = L.o[0] - a.x, x1 = L.o[1] - a.y, x2 = L.o[2] - a.z;
                 const double q = fma(x0, L.d[0], fma(x1, L.d[1], x2 * L.d[2]));
@@ -685,7 +709,7 @@ struct Walker {
                 bool certain = false;
                 if (disc >= 2.0 * Edisc) {
                     float Et;
-                    const float b = (float)-q, t = b - certain_sqrt(b, (float)disc, r, Et);
+                    const float b = (float)-q, t = b - certain_sqrt(b, (float)disc, (float)Ep, (float)Edisc, Et);
                     if (t < -2.0f * Et || t - Et > U) continue;        // no entry ahead, or behind the best one
                     certain = t > Et;
                 }
@@ -697,31 +721,45 @@ struct Walker {
                     U = __double2float_ru(best);
                 }
             } else {
-                float4 a = __ldg(S.atoms + k);
-                float vx = a.x - r.ox, vy = a.y - r.oy, vz = a.z - r.oz;
-                float b = fmaf(vx, r.dx, fmaf(vy, r.dy, vz * r.dz));
-                // the short discriminant; r.Edisc is widened for it (kWidenShortDisc)
-                float w = fmaf(-vx, vx, fmaf(-vy, vy, fmaf(-vz, vz, a.w * a.w)));
-                float disc = fmaf(b, b, w);
-                if (disc < -r.Edisc || b < -r.Ep) continue;
+                const float4 a = __ldg(S.atoms + k);
+                float b;
+                const float D = sphere_disc(r, a, b);
+                if (D < r.thr || b < r.bmin) continue;
                 // the start atom is excluded after the cheap reject, which a ray leaving that
                 // atom's surface (moving away from its centre) nearly always takes
                 if (k == last_rank) continue;
-                if (disc >= 2.0f * r.Edisc) {
+                const float Edisc = ray_edisc(S.h), Ep = ray_ep(S.h);
+                const float disc = fmaf(2.0f, D - r.thr, -Edisc), bt = fmaf(b - r.bmin, kSqrt2, -Ep);
+                if (disc >= 2.0f * Edisc) {
                     float Et;
-                    const float t = b - certain_sqrt(b, disc, r, Et);
+                    const float t = bt - certain_sqrt(bt, disc, Ep, Edisc, Et);
                     if (t < -2.0f * Et) continue;
                     if (t > Et) {
-                        float up = t + Et;
+                        const float up = t + Et;
                         if (up < U) U = up;
                         add_candidate(k, t - Et);
                         continue;
                     }
                 }
                 grazing = true;
-                add_candidate(k, fmaxf(0.0f, (b - r.Ep - sqrtf(fmaxf(disc, 0.0f) + r.Edisc)) * (1.0f - 8.0f * kU32)));
+                add_candidate(k, fmaxf(0.0f, (bt - Ep - sqrtf(fmaxf(disc, 0.0f) + Edisc)) * (1.0f - 8.0f * kU32)));
             }
         }
+    }
+    // The ray of a new query.  Not kRayOk: a query for the out-of-line search (an origin beyond the walk's bounds, or
+    // for FILTER a direction that is not unit).
+    __device__ __forceinline__ int start(const SceneHeader* H, const LaneRay& L) {
+        reset();
+        const int kind = setup_ray(H, L.o, L.d, r);
+        if (!EXACT || kind == kRayFar) return kind;
+        r.thr = kind == kRayOk ? 0.0f : CUDART_INF_F;
+        return kRayOk;
+    }
+    // No lane of the warp is in a query: nothing of it has to be kept across a call.
+    __device__ __forceinline__ void forget() {
+        reset();
+        r = RayF{0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+        best = 0.; best_rank = best_id = -1;
     }
 };
 
@@ -744,6 +782,32 @@ __device__ __forceinline__ int resolve_candidates(const SceneView& S, const Walk
         }
     }
     return k;
+}
+
+// The rest of a parked ray's path, from its current query on, in FP64.  A lane parks its ray when the query overflows its candidate slots
+// (one in 450,000 on the mixed 256-globule batch) or cannot be walked in FP32,
+// and the warp takes the parked rays when no lane is in a query: as a call in the
+// resolve phase, every value that a lane holds across it was stored and
+// reloaded on the hot path (88 / 116 B of spills a thread, 10 % of the batched
+// trace).  Inlined here, where no value of a query is live; as a call it still
+// cost 4 %.  Returns whether the ray escaped.
+__device__ __forceinline__ bool rest_of_path(const void* scene, LaneRay& L, int cap, int& bounces, int& last_rank,
+                                          int32_t* history, LocalStats& st) {
+    const SceneView S = scene_view(scene);
+    bool first = true;
+    while (true) {
+        double best;
+        const int k = nearest<true>(S, L.o, L.d, last_rank, best, st);
+        if (first) --st.queries;                          // counted when the query began
+        first = false;
+        if (k < 0) return true;
+        if (bounces >= cap) return false;
+        const double4 a = S.atoms64[k];
+        reflect64(L.o[0], L.o[1], L.o[2], L.d[0], L.d[1], L.d[2], a.x, a.y, a.z, a.w, best);
+        if (history) history[bounces] = S.ids[k];
+        ++bounces;
+        last_rank = k;
+    }
 }
 
 // Rare path of k_blocks, kept out of line so that it costs the hot loop no registers.
@@ -840,6 +904,18 @@ __global__ void __launch_bounds__(128, 8) k_blocks(const ehss_block* blocks, int
         int pool = 0, bounces = 0, last_rank = -1;
         while (true) {
             // ---- resolve finished queries (FP64) ----
+            if (PA && !RAYS && status == kDone && bounces == 0 && (W.grazing || W.overflow) &&
+                (__ldg(&B->flags) & EHSS_BLOCK_PA)) {
+                // a near-tangent first query leaves PA (below) to the any-hit query
+                LocalStats pst;
+                if (anyhit(scene_view(sbase), L.o, L.d, -1, pst)) atomicAdd(&A.pa, 1u);
+                if (COUNT) { W.box += pst.box; W.sphere += pst.sphere; }
+            }
+            if (!EXACT && status == kDone && W.overflow && !W.error) {
+                if (W.grazing) atomicAdd(&A.grazing, 1u);
+                atomicAdd(&A.fallback, 1u);
+                status = kParked;                         // rest_of_path
+            }
             if (status == kDone) {
                 const SceneView S = scene_view(sbase);
                 int k;
@@ -852,29 +928,15 @@ __global__ void __launch_bounds__(128, 8) k_blocks(const ehss_block* blocks, int
                     atomicAdd(&A.fp64, 1u);
                 } else {
                     if (W.grazing) atomicAdd(&A.grazing, 1u);
-                    if (W.overflow) {
-                        LocalStats fst;
-                        k = nearest<true>(S, L.o, L.d, last_rank, best, fst);
-                        atomicAdd(&A.fallback, 1u);
-                        atomicAdd(&A.fp64, fst.fp64);
-                    } else {
-                        unsigned f = 0;
-                        k = resolve_candidates<COUNT>(S, reinterpret_cast<const Walker<false, COUNT>&>(W), L, best, f);
-                        atomicAdd(&A.fp64, f);
-                    }
+                    unsigned f = 0;
+                    k = resolve_candidates<COUNT>(S, reinterpret_cast<const Walker<false, COUNT>&>(W), L, best, f);
+                    atomicAdd(&A.fp64, f);
                 }
                 // PA of a ray that is traced too: its first query has met a sphere for certain or missed every one
-                // for certain, unless a test was near-tangent (such a ray asks the any-hit query).  Disk rays start
-                // outside every sphere, where "meets" and "enters" agree.
-                if (PA && !RAYS && bounces == 0 && (__ldg(&B->flags) & EHSS_BLOCK_PA)) {
-                    bool blocked = k >= 0;
-                    if (W.grazing || W.overflow) {
-                        LocalStats pst;
-                        blocked = anyhit(S, L.o, L.d, -1, pst);
-                        if (COUNT) { W.box += pst.box; W.sphere += pst.sphere; }
-                    }
-                    if (blocked) atomicAdd(&A.pa, 1u);
-                }
+                // for certain, unless a test was near-tangent.  Disk rays start outside every sphere, where "meets"
+                // and "enters" agree.
+                if (PA && !RAYS && bounces == 0 && k >= 0 && !W.grazing && (__ldg(&B->flags) & EHSS_BLOCK_PA))
+                    atomicAdd(&A.pa, 1u);
                 if (k < 0 || bounces >= __ldg(&B->cap)) {
                     bool escaped = k < 0;
                     unsigned long long fx = 0;
@@ -906,8 +968,7 @@ __global__ void __launch_bounds__(128, 8) k_blocks(const ehss_block* blocks, int
                     reflect64(L.o[0], L.o[1], L.o[2], L.d[0], L.d[1], L.d[2], a.x, a.y, a.z, a.w, best);
                     ++bounces;
                     last_rank = k;
-                    W.reset();
-                    if (!(EXACT ? setup_exact(S.h, L.o, L.d, W.r) : setup_ray(S.h, L.o, L.d, W.r, kWidenShortDisc))) W.error = true;   // bounce points lie within S
+                    W.error = W.start(S.h, L) != kRayOk;     // bounce points lie within S, directions are unit
                     atomicAdd(&A.queries, 1u);
                     status = kTraverse;
                 }
@@ -950,10 +1011,11 @@ __global__ void __launch_bounds__(128, 8) k_blocks(const ehss_block* blocks, int
                         bounces = 0;
                         last_rank = -1;
                         if (__ldg(&B->flags) & EHSS_BLOCK_EHSS) {
-                            W.reset();
-                            if (!(EXACT ? setup_exact(S.h, L.o, L.d, W.r) : setup_ray(S.h, L.o, L.d, W.r, kWidenShortDisc))) W.error = true;
+                            const int kind = W.start(S.h, L);
+                            W.error = kind == kRayFar;
                             atomicAdd(&A.queries, 1u);
                             status = kTraverse;
+                            if (!EXACT && kind == kRayNotUnit) { atomicAdd(&A.fallback, 1u); status = kParked; }
                         }
                     } else {
                         status = kIdle;
@@ -962,7 +1024,38 @@ __global__ void __launch_bounds__(128, 8) k_blocks(const ehss_block* blocks, int
                 pool += __popc(need);
                 if (__any_sync(0xffffffffu, status == kNeedRay)) continue;   // PA-only lanes refill again
             }
-            if (!__any_sync(0xffffffffu, status == kTraverse)) break;
+            if (!__any_sync(0xffffffffu, status == kTraverse)) {
+                if (EXACT || !__any_sync(0xffffffffu, status == kParked)) break;
+                // ---- parked rays ----
+                if (status == kParked) {
+                    LocalStats st;
+                    int count = bounces, last = last_rank;      // copies: the variables stay in registers
+                    const bool escaped = rest_of_path(sbase, L, __ldg(&B->cap), count, last, nullptr, st);
+                    bounces = count;
+                    last_rank = last;
+                    atomicAdd(&A.queries, st.queries);
+                    atomicAdd(&A.grazing, st.grazing);
+                    atomicAdd(&A.fallback, st.fallback);
+                    atomicAdd(&A.fp64, st.fp64);
+                    atomicAdd(&A.errors, st.errors);
+                    if (COUNT) { W.box += st.box; W.sphere += st.sphere; }
+                    status = kDone;                       // without candidates: escaped
+                    if (!escaped) {
+                        atomicAdd(&A.unresolved, 1u);
+                        atomicAdd(&A.hits, 1u);
+                        if (RAYS) {
+                            atomicAdd(&A.unres_fx, __double2ull_rn(*rho_lane * kFxScale));
+                            atomicAdd(&A.hits_fx, __double2ull_rn(*rho_lane * kFxScale));
+                        }
+                        if (residual) save_residual(residual, residual_capacity, residual_count, L, bi, last_rank, bounces);
+                        if (bounces < kSmemBins) atomicAdd(&A.count[bounces], 1u);
+                        else atomicAdd((unsigned long long*)&hist[B->hist_offset + bounces], 1ull);
+                        status = kNeedRay;
+                    }
+                }
+                W.forget();
+                continue;
+            }
             // ---- traverse until enough queries are finished ----
             const SceneView S = scene_view(sbase);
             while (true) {
@@ -980,13 +1073,9 @@ __global__ void __launch_bounds__(128, 8) k_blocks(const ehss_block* blocks, int
                     }
                     if (W.leaf != kNoLeaf) {
                         W.leaf_tests(S, W.leaf, last_rank, L);
-                        W.leaf = kNoLeaf;
-                        if (W.cur < 0) {
-                            W.leaf = W.cur;
-                            W.cur = W.pop(smem_stack);
-                        }
+                        W.next_leaf(smem_stack);
                     }
-                    if (W.cur == kSentinel && W.leaf == kNoLeaf) status = kDone;
+                    if (W.finished()) status = kDone;
                 }
                 // lanes waiting for a new ray count towards the resolve batch
                 unsigned done = __ballot_sync(0xffffffffu, status == kDone || status == kNeedRay);
@@ -1080,8 +1169,16 @@ __device__ __forceinline__ void export_bytes(void* dst, const void* src, int64_t
     for (int64_t i = begin + lane; i < end; i += 32) d[i] = __ldcg(s + i);
 }
 
+__device__ __forceinline__ void store_result(const RayCall& C, const LaneRay& L, int64_t ray, int bounces, bool escaped) {
+#pragma unroll
+    for (int c = 0; c < 3; ++c) { C.Po[3 * ray + c] = L.o[c]; C.Do[3 * ray + c] = L.d[c]; }
+    C.bounces_out[ray] = bounces;
+    C.escaped[ray] = escaped;
+    C.unresolved[ray] = !escaped;
+}
+
 // Counts the warp's finished rays; runs that are complete with them go to the host.
-__device__ __noinline__ void export_runs(const RayCall& C, bool fin, int64_t ray) {
+__device__ __forceinline__ void export_runs(const RayCall& C, bool fin, int64_t ray) {
     bool last_of_run = false;
     if (fin) {
         const int64_t g = ray / kExportRays;
@@ -1123,23 +1220,18 @@ __global__ void __launch_bounds__(128, kRayCtas) k_rays(const __grid_constant__ 
     while (true) {
         // ---- resolve finished queries (FP64) ----
         bool fin = false;
+        if (!EXACT && status == kDone && W.overflow && !W.error) {
+            if (W.grazing) atomicAdd(&A.grazing, 1u);
+            atomicAdd(&A.fallback, 1u);
+            status = kParked;                             // rest_of_path
+        }
         if (status == kDone) {
             const SceneView S = scene_view(C.scene);
             int k;
             double best;
-            const bool far = W.steps < 0;             // origin beyond the FP32 bounds: all-atom search
             if (W.error) {
                 atomicAdd(&A.errors, 1u);
                 k = -1; best = CUDART_INF;
-            } else if (far || (!EXACT && W.overflow)) {
-                if (!EXACT && W.grazing) atomicAdd(&A.grazing, 1u);
-                LocalStats fst;
-                k = nearest<true>(S, L.o, L.d, last_rank, best, fst);
-                if (!far) atomicAdd(&A.fallback, 1u);
-                if (!EXACT) atomicAdd(&A.fp64, fst.fp64);
-                if (fst.errors) atomicAdd(&A.errors, fst.errors);
-                W.box += fst.box;
-                W.sphere += fst.sphere;
             } else if (EXACT) {
                 k = W.best_rank; best = W.best;
             } else {
@@ -1149,11 +1241,7 @@ __global__ void __launch_bounds__(128, kRayCtas) k_rays(const __grid_constant__ 
                 atomicAdd(&A.fp64, f);
             }
             if (k < 0 || bounces >= C.cap) {
-#pragma unroll
-                for (int c = 0; c < 3; ++c) { C.Po[3 * ray + c] = L.o[c]; C.Do[3 * ray + c] = L.d[c]; }
-                C.bounces_out[ray] = bounces;
-                C.escaped[ray] = k < 0;
-                C.unresolved[ray] = k >= 0;
+                store_result(C, L, ray, bounces, k < 0);
                 fin = true;
                 status = kNeedRay;
             } else {
@@ -1162,10 +1250,8 @@ __global__ void __launch_bounds__(128, kRayCtas) k_rays(const __grid_constant__ 
                 if (C.history) C.history[ray * (int64_t)C.cap + bounces] = S.ids[k];
                 ++bounces;
                 last_rank = k;
-                W.reset();
-                if (!(EXACT ? setup_exact(S.h, L.o, L.d, W.r) : setup_ray(S.h, L.o, L.d, W.r, kWidenShortDisc))) { W.steps = -1; W.cur = kSentinel; }
+                status = W.start(S.h, L) == kRayOk ? kTraverse : kParked;
                 atomicAdd(&A.queries, 1u);
-                status = kTraverse;
             }
         }
         if (C.finished && __any_sync(full, fin)) export_runs(C, fin, ray);
@@ -1221,10 +1307,8 @@ __global__ void __launch_bounds__(128, kRayCtas) k_rays(const __grid_constant__ 
                         if (C.history && count == 1) C.history[ray * (int64_t)C.cap] = (int32_t)last_id;
                         bounces = (int)count;
                         last_rank = last_id >= 0 ? S.rank[last_id] : -1;
-                        W.reset();
-                        if (!(EXACT ? setup_exact(S.h, L.o, L.d, W.r) : setup_ray(S.h, L.o, L.d, W.r, kWidenShortDisc))) { W.steps = -1; W.cur = kSentinel; }
+                        status = W.start(S.h, L) == kRayOk ? kTraverse : kParked;
                         atomicAdd(&A.queries, 1u);
-                        status = kTraverse;
                     }
                 }
             }
@@ -1232,6 +1316,30 @@ __global__ void __launch_bounds__(128, kRayCtas) k_rays(const __grid_constant__ 
         }
         if (C.finished && __any_sync(full, bad)) export_runs(C, bad, ray);
         if (!__any_sync(full, status == kTraverse)) {
+            if (__any_sync(full, status == kParked)) {
+                // ---- parked rays ----
+                const bool parked = status == kParked;
+                if (parked) {
+                    LocalStats st;
+                    int count = bounces, last = last_rank;      // copies: the variables stay in registers
+                    const bool out = rest_of_path(C.scene, L, C.cap, count, last,
+                                                         C.history ? C.history + ray * (int64_t)C.cap : nullptr, st);
+                    bounces = count;
+                    last_rank = last;
+                    atomicAdd(&A.queries, st.queries);
+                    atomicAdd(&A.grazing, st.grazing);
+                    atomicAdd(&A.fallback, st.fallback);
+                    if (!EXACT) atomicAdd(&A.fp64, st.fp64);
+                    atomicAdd(&A.errors, st.errors);
+                    W.box += st.box;
+                    W.sphere += st.sphere;
+                    store_result(C, L, ray, bounces, out);
+                    status = kNeedRay;
+                }
+                W.forget();
+                if (C.finished) export_runs(C, parked, ray);
+                continue;
+            }
             if (!__any_sync(full, status == kNeedRay)) break;
             continue;
         }
@@ -1240,7 +1348,7 @@ __global__ void __launch_bounds__(128, kRayCtas) k_rays(const __grid_constant__ 
         while (true) {
             if (status == kTraverse) {
                 W.advance(S, smem_stack, last_rank, L);
-                if (W.cur == kSentinel && W.leaf == kNoLeaf) status = kDone;
+                if (W.finished()) status = kDone;
             }
             // lanes without a ray count towards the batch: the call's last rays do not wait for one another
             const unsigned trav = __ballot_sync(full, status == kTraverse);
@@ -1392,7 +1500,8 @@ __global__ void __launch_bounds__(128) k_extend(const ehss_block* blocks, int nb
         int s_last = last_rank;
         while (true) {
             double best;
-            const int k = exact ? nearest<true>(S, o, d, last_rank, best, st) : nearest<false>(S, o, d, last_rank, best, st);
+            const int k = exact ? nearest_call<true>(S, o, d, last_rank, best, st)
+                                : nearest_call<false>(S, o, d, last_rank, best, st);
             if (k < 0) { escaped = true; break; }
             if (count >= new_cap) {
                 for (int c = 0; c < 3; ++c) { so[c] = o[c]; sd[c] = d[c]; }
