@@ -114,19 +114,68 @@ __device__ __forceinline__ double ddiv(double a, double b) { return __ddiv_rn(a,
 __device__ __forceinline__ double dsqrt(double a) { return __dsqrt_rn(a); }
 __device__ __forceinline__ double dmax0(double a) { return a > 0. ? a : 0.; }
 
+// Correctly rounded quotients by one denominator, for the three components of a
+// normalisation and the two quotients by d.d of the entry formula.  With
+// y = RN(1/b) and q0 within one ulp of a/b, q = RN(q0 + y (a - b q0)) is RN(a/b)
+// (Markstein 1990; the residual is exact); q0 = RN(a y + RN(a w)) with
+// w = (1 - b y) y is within (1/2 + 2^-50) ulp.  Four operations a quotient
+// after the reciprocal; a division on its own takes about eleven (256 globules:
+// 21.8 -> 20.9 ms; in FP64, 48 globules, 6.31 -> 5.91 ms).  Exact for
+// numerators that are zero or above 2^-900 in magnitude and denominators within
+// 2^-900 .. 2^900 (the residual's last place must not underflow).
+struct Denominator {
+    double b, y, w;
+};
+
+__device__ __forceinline__ Denominator denominator(double b, double y) {
+    Denominator D;
+    D.b = b;
+    D.y = y;
+    D.w = __dmul_rn(__fma_rn(-b, y, 1.0), y);
+    return D;
+}
+
+__device__ __forceinline__ double quotient(double a, const Denominator& D) {
+    const double q0 = __fma_rn(a, D.y, __dmul_rn(a, D.w));
+    const double q = __fma_rn(__fma_rn(-D.b, q0, a), D.y, q0);
+    return a == 0. ? a : q;                               // keeps the zero's sign (b > 0)
+}
+
+__device__ __forceinline__ void divide3(double& v0, double& v1, double& v2, const Denominator& D) {
+    v0 = quotient(v0, D); v1 = quotient(v1, D); v2 = quotient(v2, D);
+}
+
+// b within 2^-30 of 1 (the squared length of a unit vector, and its length):
+// with b = 1 + e, e exact, the reciprocal and the square root round like 1 - e
+// and 1 + e/2 moved a little to the side of the next term of their series, which
+// decides the ties (e is a whole number of last places, e/2 of half ones; the
+// next terms, e^2 and -e^2/8, and the shifts, below |e| 2^-29, stay under a
+// quarter of the last place).
+__device__ __forceinline__ double rcp_near_one(double b) { return __fma_rn(__dsub_rn(1.0, b), 1.0 + 0x1p-30, 1.0); }
+__device__ __forceinline__ double sqrt_near_one(double b) {
+    const double e = __dsub_rn(b, 1.0);
+    return __fma_rn(e, e < 0. ? 0.5 + 0x1p-31 : 0.5 - 0x1p-31, 1.0);
+}
+
 // entry_scalar (src/support_exchange_transport/ehss_cpu.py:12-24) ==
 // entry_distance (ehss_reference.py:8-23) == entry (src/native/ehss_cpu.cpp:7-17).
+// UNIT: |d|^2 is within 2^-30 of 1 (disk rays and their reflections: within a few last places).
+template <bool UNIT = false>
 __device__ __forceinline__ double entry64(double o0, double o1, double o2, double d0, double d1, double d2,
                                           double c0, double c1, double c2, double radius) {
     double x0 = dsub(o0, c0), x1 = dsub(o1, c1), x2 = dsub(o2, c2);
     double aa = dadd(dadd(dmul(d0, d0), dmul(d1, d1)), dmul(d2, d2));
-    double projection = ddiv(dadd(dadd(dmul(x0, d0), dmul(x1, d1)), dmul(x2, d2)), aa);
+    const double dot = dadd(dadd(dmul(x0, d0), dmul(x1, d1)), dmul(x2, d2));
+    Denominator A;
+    if (UNIT) A = denominator(aa, rcp_near_one(aa));
+    const double projection = UNIT ? quotient(dot, A) : ddiv(dot, aa);
     double p0 = dsub(x0, dmul(projection, d0));
     double p1 = dsub(x1, dmul(projection, d1));
     double p2 = dsub(x2, dmul(projection, d2));
     double disc = dsub(dmul(radius, radius), dadd(dadd(dmul(p0, p0), dmul(p1, p1)), dmul(p2, p2)));
     if (disc < 0. || projection >= 0.) return CUDART_INF;
-    double near_ = dsub(-projection, dsqrt(ddiv(dmax0(disc), aa)));
+    disc = dmax0(disc);
+    double near_ = dsub(-projection, dsqrt(UNIT ? quotient(disc, A) : ddiv(disc, aa)));
     if (near_ < dmul(-64.0 * DBL_EPSILON, radius)) return CUDART_INF;
     return dmax0(near_);
 }
@@ -142,19 +191,27 @@ __device__ __forceinline__ bool sphere_hit64(double o0, double o1, double o2, do
 }
 
 // reflect_scalar (ehss_cpu.py:27-40) == reflect (src/native/ehss_cpu.cpp:31-40).
+template <bool UNIT = false>
 __device__ __forceinline__ void reflect64(double& o0, double& o1, double& o2, double& d0, double& d1, double& d2,
                                           double c0, double c1, double c2, double r, double distance) {
     double n0 = dsub(dadd(o0, dmul(distance, d0)), c0);
     double n1 = dsub(dadd(o1, dmul(distance, d1)), c1);
     double n2 = dsub(dadd(o2, dmul(distance, d2)), c2);
     double norm = dsqrt(dadd(dadd(dmul(n0, n0), dmul(n1, n1)), dmul(n2, n2)));
-    n0 = ddiv(n0, norm); n1 = ddiv(n1, norm); n2 = ddiv(n2, norm);
+    if (UNIT) divide3(n0, n1, n2, denominator(norm, __drcp_rn(norm)));
+    else { n0 = ddiv(n0, norm); n1 = ddiv(n1, norm); n2 = ddiv(n2, norm); }
     o0 = dadd(c0, dmul(r, n0)); o1 = dadd(c1, dmul(r, n1)); o2 = dadd(c2, dmul(r, n2));
     double dot = dadd(dadd(dmul(d0, n0), dmul(d1, n1)), dmul(d2, n2));
     double two_dot = dmul(2.0, dot);
     d0 = dsub(d0, dmul(two_dot, n0)); d1 = dsub(d1, dmul(two_dot, n1)); d2 = dsub(d2, dmul(two_dot, n2));
-    norm = dsqrt(dadd(dadd(dmul(d0, d0), dmul(d1, d1)), dmul(d2, d2)));
-    d0 = ddiv(d0, norm); d1 = ddiv(d1, norm); d2 = ddiv(d2, norm);
+    const double dd = dadd(dadd(dmul(d0, d0), dmul(d1, d1)), dmul(d2, d2));
+    if (UNIT) {
+        norm = sqrt_near_one(dd);
+        divide3(d0, d1, d2, denominator(norm, rcp_near_one(norm)));
+    } else {
+        norm = dsqrt(dd);
+        d0 = ddiv(d0, norm); d1 = ddiv(d1, norm); d2 = ddiv(d2, norm);
+    }
 }
 
 // clip(1 - incoming . outgoing, 0, 2) of EHSSResult.contributions
@@ -206,7 +263,7 @@ __device__ __forceinline__ Ray64 impact_ray(uint4 q, const double* center, doubl
     double t1 = dsub(dmul(a2, d0), dmul(a0, d2));
     double t2 = dsub(dmul(a0, d1), dmul(a1, d0));
     double tn = dsqrt(dadd(dadd(dmul(t0, t0), dmul(t1, t1)), dmul(t2, t2)));
-    t0 = ddiv(t0, tn); t1 = ddiv(t1, tn); t2 = ddiv(t2, tn);
+    divide3(t0, t1, t2, denominator(tn, __drcp_rn(tn)));   // tn >= .43
     double b0 = dsub(dmul(d1, t2), dmul(d2, t1));
     double b1 = dsub(dmul(d2, t0), dmul(d0, t2));
     double b2 = dsub(dmul(d0, t1), dmul(d1, t0));

@@ -29,6 +29,7 @@
 //     re-runs the query in EXACT mode.
 // Ray origins farther than 3 S from the structure centre (never produced by
 // the impact-disk source) use an FP64 all-atom search instead.
+#include <algorithm>
 #include <cstdio>
 #include "ehss_internal.cuh"
 
@@ -594,7 +595,8 @@ constexpr int kNoLeaf = INT32_MAX;
 // per-lane local array.
 constexpr int kSmemStackMax = 32;
 
-template <bool EXACT, bool COUNT>
+// UNIT: every ray's direction is unit to rounding (disk rays).
+template <bool EXACT, bool COUNT, bool UNIT>
 struct Walker {
     RayF r;
     float U;
@@ -691,7 +693,7 @@ struct Walker {
         if (first + cnt > S.h->n_atoms) { error = true; return; }
         if (COUNT) sphere += cnt - ((unsigned)(last_rank - first) < (unsigned)cnt ? 1 : 0);
         // EXACT: the FP64 reject takes |d| = 1 and is off (infinite bounds) for other directions
-        const double slack = EXACT ? (r.thr == CUDART_INF_F ? CUDART_INF : 1.0) : 0.;
+        const double slack = EXACT ? (!UNIT && r.thr == CUDART_INF_F ? CUDART_INF : 1.0) : 0.;
         const double Edisc = EXACT ? ray_edisc(S.h) * slack : 0., Ep = EXACT ? ray_ep(S.h) * slack : 0.;
         for (int k = first; k < first + cnt; ++k) {
             if (EXACT) {
@@ -714,7 +716,7 @@ struct Walker {
                     certain = t > Et;
                 }
                 if (!certain) grazing = true;
-                const double t = entry64(L.o[0], L.o[1], L.o[2], L.d[0], L.d[1], L.d[2], a.x, a.y, a.z, a.w);
+                const double t = entry64<UNIT>(L.o[0], L.o[1], L.o[2], L.d[0], L.d[1], L.d[2], a.x, a.y, a.z, a.w);
                 const int id = __ldg(S.ids + k);
                 if (better(t, id, best, best_id)) {
                     best = t; best_rank = k; best_id = id;
@@ -765,8 +767,8 @@ struct Walker {
 
 // FP64 resolution of a finished FILTER query: re-test the candidates with the
 // reference formula and the (distance, id) rule.
-template <bool COUNT>
-__device__ __forceinline__ int resolve_candidates(const SceneView& S, const Walker<false, COUNT>& W, const LaneRay& L,
+template <bool COUNT, bool UNIT>
+__device__ __forceinline__ int resolve_candidates(const SceneView& S, const Walker<false, COUNT, UNIT>& W, const LaneRay& L,
                                                   double& best, unsigned& fp64) {
     best = CUDART_INF;
     int k = -1, best_id = -1;
@@ -775,7 +777,7 @@ __device__ __forceinline__ int resolve_candidates(const SceneView& S, const Walk
         if (W.cand_rank[e] >= 0 && W.cand_lo[e] <= W.U) {
             int kk = W.cand_rank[e];
             double4 a = S.atoms64[kk];
-            double t = entry64(L.o[0], L.o[1], L.o[2], L.d[0], L.d[1], L.d[2], a.x, a.y, a.z, a.w);
+            double t = entry64<UNIT>(L.o[0], L.o[1], L.o[2], L.d[0], L.d[1], L.d[2], a.x, a.y, a.z, a.w);
             ++fp64;
             int id = __ldg(S.ids + kk);
             if (better(t, id, best, best_id)) { best = t; k = kk; best_id = id; }
@@ -864,7 +866,7 @@ __global__ void __launch_bounds__(128, 8) k_blocks(const ehss_block* blocks, int
     // RAYS: each lane's ray weight relative to the block's largest, after the stack
     double* rho_lane = reinterpret_cast<double*>(stack_base + smem_stack * blockDim.x) + threadIdx.x;
     const unsigned lt_mask = (1u << lane) - 1u;
-    Walker<EXACT, COUNT> W;
+    Walker<EXACT, COUNT, !RAYS> W;
     int scan = 0;
     while (true) {
         long long c = 0;
@@ -929,7 +931,7 @@ __global__ void __launch_bounds__(128, 8) k_blocks(const ehss_block* blocks, int
                 } else {
                     if (W.grazing) atomicAdd(&A.grazing, 1u);
                     unsigned f = 0;
-                    k = resolve_candidates<COUNT>(S, reinterpret_cast<const Walker<false, COUNT>&>(W), L, best, f);
+                    k = resolve_candidates(S, reinterpret_cast<const Walker<false, COUNT, !RAYS>&>(W), L, best, f);
                     atomicAdd(&A.fp64, f);
                 }
                 // PA of a ray that is traced too: its first query has met a sphere for certain or missed every one
@@ -965,7 +967,7 @@ __global__ void __launch_bounds__(128, 8) k_blocks(const ehss_block* blocks, int
                     status = kNeedRay;
                 } else {
                     double4 a = S.atoms64[k];
-                    reflect64(L.o[0], L.o[1], L.o[2], L.d[0], L.d[1], L.d[2], a.x, a.y, a.z, a.w, best);
+                    reflect64<!RAYS>(L.o[0], L.o[1], L.o[2], L.d[0], L.d[1], L.d[2], a.x, a.y, a.z, a.w, best);
                     ++bounces;
                     last_rank = k;
                     W.error = W.start(S.h, L) != kRayOk;     // bounce points lie within S, directions are unit
@@ -1145,8 +1147,9 @@ struct RayCall {
     uint8_t *escaped, *unresolved;
     int32_t* history;
     uint64_t* stats;
-    unsigned long long* next;          // rays handed out; NULL: warps take fixed runs of 32 in turn
+    unsigned long long* next;          // rays handed out; NULL: warps take fixed runs of `lanes` in turn
     unsigned* finished;                // per run of kExportRays rays; NULL: results stay on the device
+    int lanes;                         // lanes of a warp that take rays
     double *hP, *hD;                   // page-locked copies of the results
     int64_t* hb;
     uint8_t *he, *hu;
@@ -1210,12 +1213,13 @@ __global__ void __launch_bounds__(128, kRayCtas) k_rays(const __grid_constant__ 
     const bool ok = H->magic == kSceneMagic && H->status == 0 && H->exterior == 0;
     if (lane == 0) A.queries = A.grazing = A.fallback = A.fp64 = A.errors = 0;
     __syncwarp();
-    Walker<EXACT, true> W;
+    Walker<EXACT, true, false> W;
     W.box = W.sphere = 0;
-    int status = kNeedRay, bounces = 0, last_rank = -1;
+    int status = lane < C.lanes ? kNeedRay : kIdle, bounces = 0, last_rank = -1;
+    const int refill_at = min(kNewRayBatch, (C.lanes + 1) / 2);
     int64_t ray = 0;
     // fixed runs (no counter): this warp's current run [pool, pool_end) and its next one
-    int64_t run = 32 * (blockIdx.x * (int64_t)nwarps + warp), pool = run, pool_end = min(run + 32, C.n);
+    int64_t run = C.lanes * (blockIdx.x * (int64_t)nwarps + warp), pool = run, pool_end = min(run + C.lanes, C.n);
     bool more = true;
     while (true) {
         // ---- resolve finished queries (FP64) ----
@@ -1237,7 +1241,7 @@ __global__ void __launch_bounds__(128, kRayCtas) k_rays(const __grid_constant__ 
             } else {
                 if (W.grazing) atomicAdd(&A.grazing, 1u);
                 unsigned f = 0;
-                k = resolve_candidates<true>(S, reinterpret_cast<const Walker<false, true>&>(W), L, best, f);
+                k = resolve_candidates(S, reinterpret_cast<const Walker<false, true, false>&>(W), L, best, f);
                 atomicAdd(&A.fp64, f);
             }
             if (k < 0 || bounces >= C.cap) {
@@ -1258,7 +1262,7 @@ __global__ void __launch_bounds__(128, kRayCtas) k_rays(const __grid_constant__ 
         // ---- new rays for lanes whose ray finished ----
         bool bad = false;
         const unsigned need = __ballot_sync(full, status == kNeedRay);
-        const bool refill = need && (__popc(need) >= kNewRayBatch || !more || !__any_sync(full, status == kTraverse));
+        const bool refill = need && (__popc(need) >= refill_at || !more || !__any_sync(full, status == kTraverse));
         int64_t base = 0;
         int got = 0;
         if (refill && more) {
@@ -1271,9 +1275,9 @@ __global__ void __launch_bounds__(128, kRayCtas) k_rays(const __grid_constant__ 
                 more = base + want < C.n;
             } else {
                 if (pool >= pool_end) {
-                    run += 32 * (int64_t)gridDim.x * nwarps;
+                    run += C.lanes * (int64_t)gridDim.x * nwarps;
                     pool = run;
-                    pool_end = min(run + 32, C.n);
+                    pool_end = min(run + C.lanes, C.n);
                 }
                 base = pool;
                 got = (int)max((int64_t)0, min((int64_t)want, pool_end - pool));
@@ -1386,8 +1390,12 @@ int launch_trace_rays(const RayBuffers& B, int precision, cudaStream_t stream) {
     C.history = B.history; C.stats = B.stats;
     C.next = B.next; C.finished = B.finished;
     C.hP = B.host_positions; C.hD = B.host_outgoing; C.hb = B.host_bounces; C.he = B.host_escaped; C.hu = B.host_unresolved;
-    // few rays: one-warp CTAs, so that they spread over the SMs
-    const int64_t warps = (B.n + 31) / 32;
+    // Few rays take few lanes of a warp, up to one warp a scheduler: a warp's lanes diverge, so fewer of them finish
+    // sooner (2000 atoms, 4096 rays: 125 us against 165; with more warps than that, 32,768 rays: 218 against 205).
+    // At least four a warp, in one-warp CTAs where warps are few.
+    const int64_t slots = (int64_t)sm_count() * 4;
+    C.lanes = (int)std::min<int64_t>(32, std::max<int64_t>(4, (B.n + slots - 1) / slots));
+    const int64_t warps = (B.n + C.lanes - 1) / C.lanes;
     const int threads = warps < 4ll * sm_count() ? 32 : 128;
     const int64_t want = (warps * 32 + threads - 1) / threads, most = (int64_t)sm_count() * kRayCtas;
     const int sdepth = 5;
