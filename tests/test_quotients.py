@@ -19,6 +19,8 @@ def fma(a, b, c):
 
 
 def quotient(a, b, y):
+    if a == 0.:
+        return a * y
     w = rn(Q(fma(-b, y, 1.0)) * Q(y))
     q0 = fma(a, y, rn(Q(a) * Q(w)))
     return fma(fma(-b, q0, a), y, q0)
@@ -48,6 +50,13 @@ def test_quotients_by_a_shared_reciprocal():
     for a, b in zip(_mantissas(rng, 40000), _mantissas(random.Random(2), 40000)):
         a, b = math.ldexp(a, rng.randint(-40, 40)) * rng.choice((1, -1)), math.ldexp(b, rng.randint(-8, 8))
         assert quotient(a, b, rn(1 / Q(b))) == a / b
+
+
+def test_zero_numerators():
+    for b in (.5, 1., 3.):
+        for a in (0., -0.):
+            assert math.copysign(1., quotient(a, b, 1 / b)) == math.copysign(1., a / b)
+    assert math.isnan(quotient(0., 0., math.inf))          # a hit point that rounds onto its centre
 
 
 @pytest.mark.parametrize('top', [64, 2 ** 22])
