@@ -9,12 +9,15 @@
 // quadtree (block_disks / block_count, pa_sparse_blocks.py:134-166) counts
 // with the exact row inequality of row_span (pa_dyadic_bitmask.py:50-61).
 //
-// Two kernels:
+// k_grid_project, then one of the two others:
 //   k_grid_project  one CTA per (direction, 1024 atoms): direction frame,
 //                   projected centres (FP64, leaf order), the CTA's extent
 //   k_grid_cover    one CTA per (direction, band of rows), one warp per 32
 //                   rows and one lane per row: the rows' pixels as a bit mask
 //                   in shared memory, counted in place
+//   k_grid_scatter  one thread per atom, where a disk spans few rows
+// Where directions are few, the CTAs of a cluster share a direction's atoms, each
+// with a mask of its own, and count the union of their masks.
 // Counts are integers, so a direction's count equals the reference's count
 // whenever the projected coordinates are the same.
 //
@@ -38,6 +41,8 @@
 // Measured (64 directions, device time of both kernels under ncu): 34 us for 650
 // atoms on a 512 grid and 179 us for 20,000 on a 1024 grid; one thread per
 // (atom, direction) with FP64 row ends and global atomics took 121 and 1005 us.
+#include <cooperative_groups.h>
+#include <algorithm>
 #include <cstdio>
 #include "ehss_internal.cuh"
 
@@ -257,8 +262,29 @@ __device__ __forceinline__ bool columns_full(const unsigned* full, int a, int b)
     return true;
 }
 
+// Adds the pixels of a CTA's mask, or of the union of the masks of a cluster of
+// `parts` CTAs that share their rows, to a direction's count.
+__device__ __forceinline__ void add_covered(unsigned* masks, int size, int parts, int part, unsigned long long* counts) {
+    int count = 0;
+    if (parts == 1) {
+        __syncthreads();
+        for (int w = threadIdx.x; w < size; w += blockDim.x) count += __popc(masks[w]);
+    } else {
+        cooperative_groups::cluster_group cluster = cooperative_groups::this_cluster();
+        cluster.sync();
+        for (int w = part * blockDim.x + threadIdx.x; w < size; w += parts * blockDim.x) {
+            unsigned v = 0u;
+            for (int q = 0; q < parts; ++q) v |= cluster.map_shared_rank(masks, q)[w];
+            count += __popc(v);
+        }
+        cluster.sync();                                      // no CTA ends while another reads its mask
+    }
+    count = __reduce_add_sync(0xffffffffu, count);
+    if ((threadIdx.x & 31) == 0 && count) atomicAdd(counts, (unsigned long long)count);
+}
+
 __global__ void __launch_bounds__(512) k_grid_cover(const void* scene, int m_max, int all_atoms, int n, int bands, int words,
-                                                    int pitch, int chunks, const double* extents, const double2* xy_all,
+                                                    int pitch, int parts, int chunks, const double* extents, const double2* xy_all,
                                                     unsigned long long* counts, double* spacing_out) {
     extern __shared__ __align__(16) unsigned char cover_smem[];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
@@ -270,7 +296,7 @@ __global__ void __launch_bounds__(512) k_grid_cover(const void* scene, int m_max
     int* const n_staged = atom + kStage;
     unsigned* const fulls = reinterpret_cast<unsigned*>(n_staged + 1);          // [nwarps][words]
     unsigned* const masks = fulls + nwarps * words;                             // [32 nwarps][pitch]
-    const int dir = blockIdx.x / bands, band = blockIdx.x % bands;
+    const int part = blockIdx.x % parts, band = blockIdx.x / parts % bands, dir = blockIdx.x / (parts * bands);
     const SceneView S = scene_view(scene);
     const int m = grid_atoms(S.h, m_max, all_atoms != 0);
     const double2* xy = xy_all + (int64_t)dir * m_max;
@@ -278,17 +304,17 @@ __global__ void __launch_bounds__(512) k_grid_cover(const void* scene, int m_max
     for (int k = 0; k < chunks; ++k) extent = fmax(extent, extents[(int64_t)dir * chunks + k]);
     extent = dmul(extent, 1.0000000001);
     const double lower = -extent, spacing = ddiv(dmul(2.0, extent), (double)n), inv = 1.0 / spacing;
-    if (spacing_out && band == 0 && threadIdx.x == 0) spacing_out[dir] = spacing;
+    if (spacing_out && band == 0 && part == 0 && threadIdx.x == 0) spacing_out[dir] = spacing;
     const int band0 = band * 32 * nwarps, row0 = band0 + 32 * warp, y = row0 + lane;
     unsigned* const row = masks + threadIdx.x * pitch;
     unsigned* const full = fulls + warp * words;             // bit c: column c is covered in all of the warp's rows
     unsigned short* const list = lists + warp * kStage;
-    for (int w = 0; w < words; ++w) row[w] = 0u;
+    for (int w = 0; w < pitch; ++w) row[w] = 0u;             // the pad too: it is counted
     for (int w = lane; w < words; w += 32) full[w] = 0u;
     // Rounds take runs of 8 atoms spread over the leaf order: a first round of kStage atoms, then twice as many as
     // before while the band's full columns drop enough of them that the rest fit the stage.
     const int runs = (m + 7) >> 3, bits = max(0, 29 - __clz(runs)), width = (runs + (1 << bits) - 1) >> bits;
-    const int places = width << bits;
+    const int places = (width << bits) / parts + (part < (width << bits) % parts);
     int drawn = 0, next = 8;                                 // atoms drawn; the full columns are formed at 8 and every quarter more
     int size = kStage / 8;
     for (int begin = 0; begin < places;) {
@@ -304,7 +330,7 @@ __global__ void __launch_bounds__(512) k_grid_cover(const void* scene, int m_max
 #pragma unroll
             for (int i = 0; i < kStageLoads; ++i) {
                 const int k = k0 + i * (int)blockDim.x;
-                j[i] = k < cnt ? 8 * spread_run(begin + (k >> 3), bits, width) + (k & 7) : m;
+                j[i] = k < cnt ? 8 * spread_run((begin + (k >> 3)) * parts + part, bits, width) + (k & 7) : m;
                 c[i] = xy[min(j[i], m - 1)];
                 r[i] = S.atoms64[min(j[i], m - 1)].w;
             }
@@ -425,11 +451,57 @@ __global__ void __launch_bounds__(512) k_grid_cover(const void* scene, int m_max
             if (2 * found <= kStage) size *= 2;
         }
     }
-    int count = 0;
-    if (y < n)
-        for (int w = 0; w < words; ++w) count += __popc(row[w]);
-    count = __reduce_add_sync(0xffffffffu, count);
-    if (lane == 0 && count) atomicAdd(counts + dir, (unsigned long long)count);
+    add_covered(masks, 32 * nwarps * pitch, parts, part, counts + dir);
+}
+
+// The same count with a thread for each atom: the atom's rows in turn, their
+// words set by shared-memory atomics, and one direction's atoms shared among
+// the `parts` CTAs of a cluster, which read one another's masks to count.
+__global__ void __launch_bounds__(512) k_grid_scatter(const void* scene, int m_max, int all_atoms, int n, int bands, int rows,
+                                                      int pitch, int parts, int chunks, const double* extents,
+                                                      const double2* xy_all, unsigned long long* counts, double* spacing_out) {
+    extern __shared__ __align__(16) unsigned char cover_smem[];
+    unsigned* const masks = reinterpret_cast<unsigned*>(cover_smem);            // [rows][pitch]
+    const int part = blockIdx.x % parts, band = blockIdx.x / parts % bands, dir = blockIdx.x / (parts * bands);
+    const SceneView S = scene_view(scene);
+    const int m = grid_atoms(S.h, m_max, all_atoms != 0), band0 = band * rows, size = rows * pitch;
+    const double2* xy = xy_all + (int64_t)dir * m_max;
+    for (int w = threadIdx.x; w < size; w += blockDim.x) masks[w] = 0u;
+    double extent = 0.;
+    for (int k = 0; k < chunks; ++k) extent = fmax(extent, extents[(int64_t)dir * chunks + k]);
+    extent = dmul(extent, 1.0000000001);
+    const double lower = -extent, spacing = ddiv(dmul(2.0, extent), (double)n), inv = 1.0 / spacing;
+    if (spacing_out && band == 0 && part == 0 && threadIdx.x == 0) spacing_out[dir] = spacing;
+    __syncthreads();
+    const int runs = (m + 7) >> 3, bits = max(0, 29 - __clz(runs)), width = (runs + (1 << bits) - 1) >> bits;
+    const int places = 8 * (width << bits);
+    for (int k = part * blockDim.x + threadIdx.x; k < places; k += parts * blockDim.x) {
+        const int j = 8 * spread_run(k >> 3, bits, width) + (k & 7);
+        if (j >= m) continue;
+        const double2 c = xy[j];
+        const double r = S.atoms64[j].w;
+        const double cx = (c.x - lower) * inv - .5, cy = (c.y - lower) * inv - .5, rp = r * inv;
+        const double flx = floor(cx), fly = floor(cy);
+        const float4 d = make_float4((float)(cx - flx), (float)(cy - fly), (float)(rp * rp), (float)rp);
+        const int2 o = make_int2((int)flx, (int)fly);
+        const int ya = max(o.y - (int)d.w - 1, band0), yb = min(o.y + (int)d.w + 2, min(band0 + rows, n) - 1);
+        for (int y = ya; y <= yb; ++y) {
+            const RowEnds R = row_ends(d, o, y);
+            if (R.rem < -R.tol) continue;
+            int2 v = make_int2(R.kl + (R.fl > 0.f), R.kr + (R.fr >= 0.f));
+            if (fminf(fabsf(R.fl), fabsf(R.fr)) <= R.e || R.rem < 4.f * R.tol) v = exact_ends(c, r, d, o, y, n, lower, spacing);
+            const int a = max(v.x, 0), b = min(v.y, n) - 1;
+            if (a > b) continue;
+            unsigned* const row = masks + (y - band0) * pitch;
+            for (int w = a >> 5; w <= b >> 5; ++w) {
+                unsigned need = ~0u;
+                if (w == a >> 5) need = ~0u << (a & 31);
+                if (w == b >> 5) need &= ~0u >> (31 - (b & 31));
+                if (need & ~row[w]) atomicOr(row + w, need);     // most pixels are covered already
+            }
+        }
+    }
+    add_covered(masks, size, parts, part, counts + dir);
 }
 
 static int64_t project_chunks(int64_t n_atoms) { return (n_atoms + kProjectAtoms - 1) / kProjectAtoms; }
@@ -458,27 +530,57 @@ int launch_grid_pa(const void* scene, int64_t n_atoms, int n_dirs, uint64_t seed
         for (int k = 0; k < 30; ++k) sob.sv[j][k] = sv[j * 30 + k];
         sob.shift[j] = shift[j];
     }
-    // Warps of a CTA (32 rows each): every CTA stages every atom of its direction, so as many as leave a CTA for four
-    // SMs in five (64 directions: two CTAs, of equal work, a direction; 20,000 atoms on a 1024 grid take 239 us with 16
-    // warps, 272 with 8, 442 with 4), down to two; fewer where the masks (33 KB a warp on an 8192 grid) would not fit.
     const int words = (n + 31) / 32, pitch = words | 1;                  // odd pitch: the rows' words spread over all banks
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    cudaLaunchConfig_t cfg = {};
+    cfg.stream = stream;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    auto launch = [&](auto kernel, int bands, int parts, int threads, unsigned smem, auto... geometry) {
+        if (smem > 48u * 1024u) {                        // held per device and context, so set where needed on each call
+            const int rc = cuda_status(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem),
+                                       "grid shared memory");
+            if (rc) return rc;
+        }
+        cfg.gridDim = dim3((unsigned)(bands * parts * n_dirs));
+        cfg.blockDim = dim3((unsigned)threads);
+        cfg.dynamicSmemBytes = smem;
+        attr[0].val.clusterDim.x = (unsigned)parts;
+        attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+        return cuda_status(cudaLaunchKernelEx(&cfg, kernel, scene, (int)n_atoms, (int)(xy_out != nullptr), n, bands, geometry...,
+                                              parts, chunks, (const double*)extents, (const double2*)xy, counts, spacing_out),
+                           "adaptive PA launch");
+    };
+    k_grid_project<<<(unsigned)chunks * n_dirs, 256, 0, stream>>>(scene, sob, (int)n_atoms, chunks, extents, xy, counts, xy_out);
+    int parts = 1;
+    // A disk of a compact structure spans about 2 n / atoms^(1/3) rows. Where that is fewer than a warp has lanes
+    // (n < 16 atoms^(1/3)), most lanes of k_grid_cover have no row and its warps, one for 32 rows, are few. Device times,
+    // cover / scatter, 1 and 64 directions: 2000 atoms on a 64 grid 206 / 20 and 218 / 24 us, 6000 on 256: 66 / 42 and
+    // 124 / 81; on the line's other side 20,000 on 512: 91 / 114 and 239 / 335, 650 on 256: 27 / 36 and 36 / 42.
+    if ((long long)n * n * n < 4096ll * n_atoms) {
+        int rows = n;
+        while (rows > 1 && 4ll * rows * pitch > 136ll * 1024) rows /= 2;
+        const int bands = n / rows;
+        // CTAs that share a direction's atoms: up to two an SM, 128 atoms each (20,000 atoms, one direction, 256 grid:
+        // 527 us with one, 69 with eight)
+        while (parts < 8 && n_atoms > 128ll * parts && (long long)n_dirs * bands * parts <= sm_count()) parts *= 2;
+        const int threads = (int)std::min<int64_t>(512, (n_atoms + 32 * parts - 1) / (32 * parts) * 32);
+        return launch(k_grid_scatter, bands, parts, threads, 4u * rows * pitch, rows, pitch);
+    }
+    // Warps of a CTA (32 rows each): every CTA stages every atom of its part of the direction, so as many as leave a CTA
+    // for five SMs (20,000 atoms on a 1024 grid, 64 directions: 179 us with 16 warps, 240 with fewer), down to two; fewer
+    // where the masks (33 KB a warp on an 8192 grid) would not fit. What SMs are left then share a direction's atoms,
+    // 256 at least to a CTA (16 directions: 228 -> 97 us; one: 279 -> 73).
     const int groups = (n + 31) / 32;
     auto bytes = [&](int warps) {
         return (unsigned)(kStage * (sizeof(float4) + sizeof(int2) + sizeof(short2) + 4) + 4 + warps * (kStage * 2 + 4 * words + 128 * pitch));
     };
     int warps = groups < 16 ? groups : 16;
-    while (warps > 2 && (bytes(warps) > 160u * 1024u || 5ll * n_dirs * (groups / warps) < 4ll * sm_count())) warps /= 2;
-    const unsigned smem = bytes(warps);
-    if (smem > 48u * 1024u) {                            // held per device and context, so set where needed on each call
-        const int rc = cuda_status(cudaFuncSetAttribute(k_grid_cover, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem),
-                                   "grid shared memory");
-        if (rc) return rc;
-    }
+    while (warps > 2 && (bytes(warps) > 160u * 1024u || 5ll * n_dirs * (groups / warps) < sm_count())) warps /= 2;
     const int bands = groups / warps;
-    k_grid_project<<<(unsigned)chunks * n_dirs, 256, 0, stream>>>(scene, sob, (int)n_atoms, chunks, extents, xy, counts, xy_out);
-    k_grid_cover<<<(unsigned)bands * n_dirs, 32 * warps, smem, stream>>>(scene, (int)n_atoms, xy_out != nullptr, n, bands,
-                                                                        words, pitch, chunks, extents, xy, counts, spacing_out);
-    return cuda_status(cudaGetLastError(), "adaptive PA launch");
+    while (parts < 8 && n_atoms > 256ll * parts && 2ll * n_dirs * bands * parts <= sm_count()) parts *= 2;
+    return launch(k_grid_cover, bands, parts, 32 * warps, bytes(warps), words, pitch);
 }
 
 }  // namespace ehss

@@ -45,3 +45,14 @@ def test_exterior_scene_counts_equal_the_full_scene(atoms, kind):
     for grid in (64, 512):
         a, b = grid_counts(full, 16, grid, 3), grid_counts(exterior, 16, grid, 3)
         assert np.array_equal(a[0], b[0]) and np.array_equal(a[1], b[1])
+
+
+# both sides of the line between the two cover kernels (grid^3 against 4096 atoms), of the number of CTAs that share a
+# direction's atoms, and one CTA a direction
+@pytest.mark.parametrize('atoms,kind,directions,grid', [
+    (2, 'dense', 4, 16), (8, 'dense', 2, 32), (9, 'dense', 2, 32), (128, 'sparse', 2, 64), (129, 'sparse', 2, 64),
+    (512, 'dense', 4, 128), (513, 'dense', 4, 128), (700, 'dense', 512, 64), (2000, 'dense', 256, 16),
+    (4096, 'dense', 2, 256), (4097, 'sparse', 2, 256), (20000, 'dense', 1, 8), (20000, 'dense', 64, 64),
+    (33000, 'sparse', 1, 512), (300000, 'sparse', 1, 1024), (2000, 'dense', 4, 1024), (257, 'dense', 1, 512)])
+def test_coarse_grids_and_shared_directions(atoms, kind, directions, grid):
+    test_counts_equal_the_oracle(atoms, kind, directions, grid)
