@@ -742,10 +742,9 @@ def main():
     if rank == 0 and world == 1 and not args.no_serve:
         serve = serving_measurement()
     if rank == 0:
-        # builder: scene index + stats, 5 tree kernels per pass (keys sorted per structure in one
-        # kernel: every structure here holds at most 8192 atoms), two passes around exposure + its
-        # fix-up; then 1 persistent trace kernel
-        launches_per_step = 2 + 5 * 2 + 2 + 1
+        # builder: two passes of one tree kernel (one CTA a structure: every structure here holds at
+        # most 8192 atoms) and the emission, the exposure test between them; then 1 persistent trace kernel
+        launches_per_step = 2 * 2 + 1 + 1
         line = {"metric": METRIC, "value": value, "unit": UNIT, "n_gpus": world, "steps": args.steps,
                 "warmup": args.warmup, "ms_per_step": total_ms / args.steps, "higher_is_better": True,
                 "scaling": "weak", "vs_baseline": None, "dtype": "f32+f64", "data": "synthetic",

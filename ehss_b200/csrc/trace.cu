@@ -38,10 +38,10 @@ namespace ehss {
 constexpr float kU32 = 5.9604645e-08f;   // 2^-24
 // Candidate slots per query.  A slot whose lower bound exceeds the current U is
 // reused, so two slots overflow only when three spheres are within the error
-// band of each other (89 of 124 M queries on the mixed 256-globule batch).  Each
+// band of each other (275 of 125 M queries on the mixed 256-globule batch).  Each
 // slot is two registers of the fused kernel, which runs at its 64-register
-// bound: 2 slots trace that batch in 27.9 ms, 3 in 28.8, 4 in 29.7, while 1
-// slot sends every grazing query to the FP64 re-run (1e5 fallbacks, 29.0 ms).
+// bound: before the shorter sphere test 2 slots traced that batch in 27.9 ms, 3 in 28.8, 4 in 29.7, while 1
+// slot sent every grazing query to the FP64 search (1e5 fallbacks, 29.0 ms).
 constexpr int kCand = 2;
 constexpr int kSmemBins = 16;
 
