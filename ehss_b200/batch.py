@@ -38,6 +38,11 @@ def summarize(values):
                 replicates=len(a))
 
 
+def _writes(tensor):
+    """Number of writes to a tensor so far; None where torch does not count them."""
+    return None if tensor.is_inference() else tensor._version
+
+
 class SceneRef:
     """A scene inside a batch buffer (what BlockPlan needs of a scene)."""
 
@@ -69,6 +74,7 @@ class BatchScenes:
         self.h_xyz = t.empty(N * 3, dtype=t.float64, pin_memory=True)
         self.h_r = t.empty(N, dtype=t.float64, pin_memory=True)
         radii = self._stage(structures, 'Finite centers (N,3) and positive finite radii required.')
+        self._device_centers = self._uploaded = None      # set by upload
         self.d_xyz = t.empty(N * 3, dtype=t.float64, device=self.device)
         self.d_r = t.empty(N, dtype=t.float64, device=self.device)
         size_of = {}
@@ -101,16 +107,22 @@ class BatchScenes:
         self._require_build_buffers()
         self.d_xyz.copy_(self.h_xyz, non_blocking=True)
         self.d_r.copy_(self.h_r, non_blocking=True)
+        # the centres of what the device holds from here on: staging again does not change them
+        self._device_centers = self._centers
+        self._uploaded = _writes(self.d_xyz)
 
     def build(self, upload=True):
         self._require_build_buffers()
         if upload:
             self.upload()
         lib = _lib.load()
-        _lib.check(lib.ehss_scenes_build_centred(len(self.scenes), self._xyz_ptrs, self._r_ptrs, self._n, self.leaf_size,
-                                                 self._scenes, self._sizes, self.ws_ptr, self.ws_bytes, self.flags,
-                                                 self._centers.ctypes.data, stream_handle(self.device)),
-                   'batched scene build')
+        args = (len(self.scenes), self._xyz_ptrs, self._r_ptrs, self._n, self.leaf_size, self._scenes, self._sizes,
+                self.ws_ptr, self.ws_bytes, self.flags)
+        if self._uploaded is not None and self._uploaded == _writes(self.d_xyz):
+            rc = lib.ehss_scenes_build_centred(*args, self._device_centers.ctypes.data, stream_handle(self.device))
+        else:       # coordinates that the caller wrote on the device: their centres are summed there
+            rc = lib.ehss_scenes_build_ex(*args, stream_handle(self.device))
+        _lib.check(rc, 'batched scene build')
 
     def drop_build_buffers(self):
         """Free the builder's workspace and the device coordinates once the
