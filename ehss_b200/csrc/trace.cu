@@ -97,7 +97,11 @@ constexpr int kRayFar = 0, kRayOk = 1, kRayNotUnit = 2;
 // FP32 copy of an FP64 ray.  kRayFar: the origin is beyond 3 S from the centre
 // (or not finite), where node boxes are not widened enough.  kRayNotUnit: the
 // direction is off by more than 1e-11 in |d|^2, which the sphere test's
-// identity does not allow (boxes still hold: o is then the ray's own origin).
+// identity does not allow (boxes still hold: o is then the ray's own origin, and
+// distances along the ray are in units of |d|, so none is taken off them: Ep in
+// such units exceeds the boxes' widening from |d| = 20 on).  UNIT: the caller's
+// directions are unit to rounding.
+template <bool UNIT = false>
 __device__ __forceinline__ int setup_ray(const SceneHeader* H, const double* o, const double* d, RayF& r) {
     const double x = o[0] - H->center[0], y = o[1] - H->center[1], z = o[2] - H->center[2];
     const float S = H->scale_f;
@@ -115,7 +119,7 @@ __device__ __forceinline__ int setup_ray(const SceneHeader* H, const double* o, 
     const float q = fmaf(r.ox, r.ox, fmaf(r.oy, r.oy, r.oz * r.oz));
     // a line beyond S passes every sphere by 1e-5 S: all tests miss
     r.thr = q > 1.00002f * S * S ? CUDART_INF_F : 0.5f * (q - kEdisc * S * S);
-    r.bmin = ((float)tau0 - kEp * S) * kHalfSqrt2;
+    r.bmin = UNIT || unit ? ((float)tau0 - kEp * S) * kHalfSqrt2 : 0.0f;
     return unit ? kRayOk : kRayNotUnit;
 }
 
@@ -234,14 +238,14 @@ __device__ __forceinline__ int nearest_flat(const SceneView& S, const double* o,
 // Nearest entry: returns the leaf-order rank of the collider (or -1) and its
 // FP64 entry distance, identical to the reference's choice.  Parked rays
 // (rest_of_path, EXACT) and the cap extension use it.
-template <bool EXACT>
+template <bool EXACT, bool UNIT = false>
 __device__ __forceinline__ int nearest(const SceneView& S, const double* o, const double* d, int last_rank,
                                     double& best_out, LocalStats& st) {
     ++st.queries;
     RayF r;
-    const int kind = setup_ray(S.h, o, d, r);
+    const int kind = setup_ray<UNIT>(S.h, o, d, r);
     if (kind == kRayFar) return nearest_flat(S, o, d, last_rank, best_out, st);
-    if (!EXACT && kind == kRayNotUnit) { --st.queries; return nearest<true>(S, o, d, last_rank, best_out, st); }
+    if (!EXACT && kind == kRayNotUnit) { --st.queries; return nearest<true, UNIT>(S, o, d, last_rank, best_out, st); }
     const float Edisc = ray_edisc(S.h), Ep = ray_ep(S.h);
     float U = CUDART_INF_F;
     double best = CUDART_INF;
@@ -335,7 +339,7 @@ __device__ __forceinline__ int nearest(const SceneView& S, const double* o, cons
         if (overflow) {
             ++st.fallback;
             --st.queries;
-            return nearest<true>(S, o, d, last_rank, best_out, st);
+            return nearest<true, UNIT>(S, o, d, last_rank, best_out, st);
         }
 #pragma unroll
         for (int e = 0; e < kCand; ++e) {
@@ -752,7 +756,7 @@ struct Walker {
     // for FILTER a direction that is not unit).
     __device__ __forceinline__ int start(const SceneHeader* H, const LaneRay& L) {
         reset();
-        const int kind = setup_ray(H, L.o, L.d, r);
+        const int kind = setup_ray<UNIT>(H, L.o, L.d, r);
         if (!EXACT || kind == kRayFar) return kind;
         r.thr = kind == kRayOk ? 0.0f : CUDART_INF_F;
         return kRayOk;
@@ -793,13 +797,14 @@ __device__ __forceinline__ int resolve_candidates(const SceneView& S, const Walk
 // reloaded on the hot path (88 / 116 B of spills a thread, 10 % of the batched
 // trace).  Inlined here, where no value of a query is live; as a call it still
 // cost 4 %.  Returns whether the ray escaped.
+template <bool UNIT>
 __device__ __forceinline__ bool rest_of_path(const void* scene, LaneRay& L, int cap, int& bounces, int& last_rank,
                                           int32_t* history, LocalStats& st) {
     const SceneView S = scene_view(scene);
     bool first = true;
     while (true) {
         double best;
-        const int k = nearest<true>(S, L.o, L.d, last_rank, best, st);
+        const int k = nearest<true, UNIT>(S, L.o, L.d, last_rank, best, st);
         if (first) --st.queries;                          // counted when the query began
         first = false;
         if (k < 0) return true;
@@ -1032,7 +1037,7 @@ __global__ void __launch_bounds__(128, 8) k_blocks(const ehss_block* blocks, int
                 if (status == kParked) {
                     LocalStats st;
                     int count = bounces, last = last_rank;      // copies: the variables stay in registers
-                    const bool escaped = rest_of_path(sbase, L, __ldg(&B->cap), count, last, nullptr, st);
+                    const bool escaped = rest_of_path<!RAYS>(sbase, L, __ldg(&B->cap), count, last, nullptr, st);
                     bounces = count;
                     last_rank = last;
                     atomicAdd(&A.queries, st.queries);
@@ -1326,7 +1331,7 @@ __global__ void __launch_bounds__(128, kRayCtas) k_rays(const __grid_constant__ 
                 if (parked) {
                     LocalStats st;
                     int count = bounces, last = last_rank;      // copies: the variables stay in registers
-                    const bool out = rest_of_path(C.scene, L, C.cap, count, last,
+                    const bool out = rest_of_path<false>(C.scene, L, C.cap, count, last,
                                                          C.history ? C.history + ray * (int64_t)C.cap : nullptr, st);
                     bounces = count;
                     last_rank = last;
