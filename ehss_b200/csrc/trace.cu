@@ -1186,6 +1186,10 @@ __device__ __forceinline__ void store_result(const RayCall& C, const LaneRay& L,
 }
 
 // Counts the warp's finished rays; runs that are complete with them go to the host.
+// The results of a run come from several warps.  Each lane's are ordered before
+// its count by the fence ahead of it; the lane whose count completes the run
+// orders them before what follows by the fence behind it, and the warp barrier
+// (a ballot or shuffle orders no memory) passes that on to the lanes that copy.
 __device__ __forceinline__ void export_runs(const RayCall& C, bool fin, int64_t ray) {
     bool last_of_run = false;
     if (fin) {
@@ -1193,11 +1197,12 @@ __device__ __forceinline__ void export_runs(const RayCall& C, bool fin, int64_t 
         const unsigned size = (unsigned)min((int64_t)kExportRays, C.n - g * kExportRays);
         __threadfence();
         last_of_run = atomicAdd(C.finished + g, 1u) + 1u == size;
+        if (last_of_run) __threadfence();
     }
+    __syncwarp();
     for (unsigned todo = __ballot_sync(0xffffffffu, last_of_run); todo; todo &= todo - 1) {
         const int64_t b = __shfl_sync(0xffffffffu, ray, __ffs(todo) - 1) / kExportRays * kExportRays;
         const int64_t e = min(b + kExportRays, C.n);
-        __threadfence();
         export_bytes(C.hP, C.Po, 24 * b, 24 * e);
         export_bytes(C.hD, C.Do, 24 * b, 24 * e);
         export_bytes(C.hb, C.bounces_out, 8 * b, 8 * e);

@@ -1,0 +1,46 @@
+"""Explicit rays whose results the kernel writes to page-locked host memory:
+they equal the results in device memory, run after run, also where several warps
+finish one run of rays; and arrays off their elements' alignment are copied."""
+import ctypes as ct
+
+import numpy as np
+import pytest
+
+from oracle import oracle as O
+
+pytestmark = pytest.mark.gpu
+
+
+def _pinned(a):
+    import torch
+    t = torch.empty(a.shape, dtype=torch.from_numpy(a).dtype, pin_memory=True)
+    t.numpy()[...] = a
+    return t.numpy()
+
+
+def _source(o, d):
+    import ehss_b200 as eb
+    n = len(o)
+    return eb.EHSSSource(o, d, d, np.ones(n), np.full(n, -1), np.zeros(n, dtype=np.int64), 'test')
+
+
+@pytest.mark.parametrize('atoms,n', [(3, 300000), (300, 60001)])
+def test_every_run_of_results_reaches_the_host(atoms, n):
+    import torch
+    import ehss_b200 as eb
+    from ehss_b200 import _lib, workloads as W
+    c, r = W.triatomic()[:2] if atoms == 3 else W.globule(atoms, 5)[:2]
+    src = O.external_source(c, r, (n - 1).bit_length(), 5)
+    o, d = src['origins'][:n].copy(), src['directions'][:n].copy()
+    prep = eb.PreparedStaticGPUEHSS(eb.Spheres(c, r, deduplicate=False))
+    P, D = torch.from_numpy(o).cuda(), torch.from_numpy(d).cuda()
+    last, b = torch.full((n,), -1, device='cuda'), torch.zeros(n, dtype=torch.int64, device='cuda')
+    esc, unres = (torch.zeros(n, dtype=torch.uint8, device='cuda') for _ in range(2))
+    _lib.check(_lib.load().ehss_trace(prep.scene.ptr, n, 32, 1, P.data_ptr(), D.data_ptr(), last.data_ptr(), b.data_ptr(),
+                                      esc.data_ptr(), unres.data_ptr(), None, None, torch.cuda.current_stream().cuda_stream))
+    want = [a.cpu().numpy() for a in (P, D, b, esc.bool(), unres.bool())]
+    source = _source(_pinned(o), _pinned(d))
+    for _ in range(10):
+        got = prep.engine.trace(source, 32)
+        for a, w in zip((got.positions, got.outgoing, got.bounces, got.escaped, got.unresolved), want):
+            assert np.array_equal(a, w)
