@@ -291,10 +291,11 @@ static HostTraceLayout host_trace_layout(int64_t n) {
     return L;
 }
 
-// Address under which kernels reach p: device memory, or page-locked host memory; 0 for anything else.
-static const void* reachable(const void* p) {
+// Address under which kernels reach p, elements of `size` bytes in device memory or page-locked host memory; 0 for
+// anything else, and for addresses that are not a multiple of the element's size.
+static const void* reachable(const void* p, size_t size) {
     cudaPointerAttributes a;
-    if (!p || cudaPointerGetAttributes(&a, p) != cudaSuccess) { cudaGetLastError(); return nullptr; }
+    if (!p || (uintptr_t)p % size || cudaPointerGetAttributes(&a, p) != cudaSuccess) { cudaGetLastError(); return nullptr; }
     return a.type == cudaMemoryTypeUnregistered ? nullptr : a.devicePointer;
 }
 
@@ -322,19 +323,19 @@ int ehss_trace_host(const void* scene_dev, int64_t n_rays, int cap, int precisio
     }
     RayBuffers B = {};
     if (n_rays > 0) {
-        B.origins = (const double*)reachable(origins);
-        B.directions = (const double*)reachable(directions);
-        B.last = (const int64_t*)reachable(last_atom);
-        B.bounces = (const int64_t*)reachable(initial_bounces);
-        B.host_positions = (double*)reachable(positions_host);
-        B.host_outgoing = (double*)reachable(outgoing_host);
-        B.host_bounces = (int64_t*)reachable(bounces_host);
-        B.host_escaped = (uint8_t*)reachable(escaped_host);
-        B.host_unresolved = (uint8_t*)reachable(unresolved_host);
+        B.origins = (const double*)reachable(origins, 8);
+        B.directions = (const double*)reachable(directions, 8);
+        B.last = (const int64_t*)reachable(last_atom, 8);
+        B.bounces = (const int64_t*)reachable(initial_bounces, 8);
+        B.host_positions = (double*)reachable(positions_host, 8);
+        B.host_outgoing = (double*)reachable(outgoing_host, 8);
+        B.host_bounces = (int64_t*)reachable(bounces_host, 8);
+        B.host_escaped = (uint8_t*)reachable(escaped_host, 1);
+        B.host_unresolved = (uint8_t*)reachable(unresolved_host, 1);
         if (!scene_dev || !workspace_dev || !B.origins || !B.directions || (last_atom && !B.last) ||
             (initial_bounces && !B.bounces) || !B.host_positions || !B.host_outgoing || !B.host_bounces ||
             !B.host_escaped || !B.host_unresolved) {
-            set_error("rays and results must lie in device or page-locked host memory");
+            set_error("rays and results must lie in device or page-locked host memory, aligned as their elements");
             return EHSS_ERR_VALUE;
         }
     }
@@ -364,6 +365,10 @@ int ehss_pa_anyhit(const void* scene_dev, int64_t n_rays, const double* origins_
     if (n_rays < 0) { set_error("negative ray count"); return EHSS_ERR_VALUE; }
     if (n_rays > 0 && (!scene_dev || !origins_dev || !directions_dev || !blocked_dev)) {
         set_error("null pointer");
+        return EHSS_ERR_VALUE;
+    }
+    if (((uintptr_t)origins_dev | (uintptr_t)directions_dev | (uintptr_t)owners_dev) % 8) {
+        set_error("rays must be aligned as their elements");
         return EHSS_ERR_VALUE;
     }
     return launch_pa_rays(scene_dev, n_rays, origins_dev, directions_dev, owners_dev, blocked_dev, stats_dev,

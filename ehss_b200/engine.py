@@ -168,6 +168,12 @@ def external_source(spheres, power, seed, scene=None):
                       np.full(n, -1), np.zeros(n, dtype=np.int64), "external impact disk")
 
 
+def _host_array(a, dtype):
+    """``a`` as a C-contiguous array whose elements lie on their own alignment,
+    as kernels need them: itself where it is one, else a copy."""
+    return np.require(a, dtype, ['C', 'A'])
+
+
 def _reachable(a, device, hold):
     """Address of a contiguous host array that kernels can read where it lies
     (page-locked memory), or of a device copy; ``hold`` keeps it alive."""
@@ -212,8 +218,8 @@ class GPUEHSSTransport:
             raise ValueError('Positive cap and zero/one initial collision required')
         start = time.perf_counter()
         n = len(source.weights)
-        origins, directions = (np.ascontiguousarray(a, dtype=np.float64) for a in (source.origins, source.directions))
-        last, bounces = (np.ascontiguousarray(a, dtype=np.int64) for a in (source.last_atom, source.initial_bounces))
+        origins, directions = (_host_array(a, np.float64) for a in (source.origins, source.directions))
+        last, bounces = (_host_array(a, np.int64) for a in (source.last_atom, source.initial_bounces))
         if origins.shape != (n, 3) or directions.shape != (n, 3) or last.shape != (n,) or bounces.shape != (n,):
             raise ValueError('One origin, direction, initial identity and bounce count per weight required')
         # A source starts without colliders (-1) and collisions as a rule.  Where its ends say so, the device traces
@@ -334,8 +340,8 @@ class SphereIndex:
         owners = getattr(source, 'owners', None)
         if owners is None:
             owners = source.last_atom
-        origins, directions = (np.ascontiguousarray(a, dtype=np.float64) for a in (source.origins, source.directions))
-        own = np.ascontiguousarray(owners, dtype=np.int64)
+        origins, directions = (_host_array(a, np.float64) for a in (source.origins, source.directions))
+        own = _host_array(owners, np.int64)
         n = len(origins)
         if origins.shape != (n, 3) or directions.shape != (n, 3) or own.shape != (n,):
             raise ValueError('One origin, direction and owner per ray required')

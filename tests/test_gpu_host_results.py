@@ -44,3 +44,44 @@ def test_every_run_of_results_reaches_the_host(atoms, n):
         got = prep.engine.trace(source, 32)
         for a, w in zip((got.positions, got.outgoing, got.bounces, got.escaped, got.unresolved), want):
             assert np.array_equal(a, w)
+
+
+def _off_by(a, k):
+    """The array in page-locked memory, k bytes behind an aligned address."""
+    import torch
+    raw = torch.empty(a.nbytes + 8, dtype=torch.uint8, pin_memory=True).numpy()
+    out = np.frombuffer(raw, dtype=a.dtype, count=a.size, offset=k).reshape(a.shape)
+    out[...] = a
+    return out
+
+
+def test_misaligned_page_locked_arrays():
+    import torch
+    import ehss_b200 as eb
+    from ehss_b200 import _lib, workloads as W
+    c, r, _ = W.globule(100, 7)
+    src = O.external_source(c, r, 10, 7)
+    o, d = src['origins'], src['directions']
+    ref = O.StaticTree(c, r, 4).trace(o, d, cap=8)
+    prep = eb.PreparedStaticGPUEHSS(eb.Spheres(c, r, deduplicate=False))
+    source = _source(o, d)
+    source.origins, source.directions = _off_by(o, 4), _off_by(d, 1)
+    assert not source.origins.flags.aligned
+    got = prep.engine.trace(source, 8)
+    for f in ('positions', 'outgoing', 'escaped', 'unresolved', 'bounces'):
+        assert np.array_equal(getattr(got, f), ref[f])
+    source.owners = _off_by(np.full(1024, -1), 4)
+    blocked = eb.SphereIndex(eb.Spheres(c, r, deduplicate=False)).query(source)[0]
+    assert np.array_equal(blocked, O.PATree(c, r, 8).query(o, d, np.full(1024, -1))[0])
+    # the library refuses such addresses instead of reading them
+    lib = _lib.load()
+    wb = ct.c_uint64()
+    _lib.check(lib.ehss_trace_host_workspace_bytes(1024, ct.byref(wb)))
+    ws = torch.empty(wb.value, dtype=torch.uint8, device='cuda')
+    out = torch.empty(1024 * 58 + 64, dtype=torch.uint8, pin_memory=True)
+    p = out.data_ptr()
+    rest = (p, p + 24576, p + 49152, p + 57344, p + 58368, None, p + 59392, ws.data_ptr(), wb.value, None)
+    good = _pinned(o).ctypes.data, _pinned(d).ctypes.data
+    for ray in ((source.origins.ctypes.data, good[1]), (good[0], source.directions.ctypes.data)):
+        assert lib.ehss_trace_host(prep.scene.ptr, 1024, 8, 1, *ray, None, None, *rest) == _lib.ERR_VALUE
+        assert lib.ehss_pa_anyhit(prep.scene.ptr, 1024, *ray, None, p, None, None) == _lib.ERR_VALUE
