@@ -255,6 +255,11 @@ class GPUEHSSTransport:
 
     def _enqueue(self, origins, directions, last, bounces, cap, record_history):
         """Enqueue one trace (no wait); returns the host arrays that it fills."""
+        # the scene's device, whichever is the thread's current one: the handle of a default stream names no device
+        with torch().cuda.device(self.scene.device):
+            return self._launch(origins, directions, last, bounces, cap, record_history)
+
+    def _launch(self, origins, directions, last, bounces, cap, record_history):
         lib, t, dev = _lib.load(), torch(), self.scene.device
         n = len(origins)
         hold = []
@@ -363,6 +368,10 @@ class SphereIndex:
 
     def _enqueue(self, origins, directions, owners):
         """Enqueue one any-hit query (no wait); returns the host arrays that it fills."""
+        with torch().cuda.device(self.scene.device):      # as in GPUEHSSTransport._enqueue
+            return self._launch(origins, directions, owners)
+
+    def _launch(self, origins, directions, owners):
         lib, t, dev = _lib.load(), torch(), self.scene.device
         n = len(origins)
         hold = []
