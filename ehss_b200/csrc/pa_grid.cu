@@ -504,6 +504,9 @@ __global__ void __launch_bounds__(512) k_grid_scatter(const void* scene, int m_m
     add_covered(masks, size, parts, part, counts + dir);
 }
 
+// Most shared memory that a CTA of k_grid_cover or k_grid_scatter is given.
+constexpr int kGridSmem = 160 * 1024;
+
 static int64_t project_chunks(int64_t n_atoms) { return (n_atoms + kProjectAtoms - 1) / kProjectAtoms; }
 
 uint64_t grid_workspace_bytes(int64_t n_atoms, int n_dirs, int n) {
@@ -538,8 +541,10 @@ int launch_grid_pa(const void* scene, int64_t n_atoms, int n_dirs, uint64_t seed
     cfg.attrs = attr;
     cfg.numAttrs = 1;
     auto launch = [&](auto kernel, int bands, int parts, int threads, unsigned smem, auto... geometry) {
-        if (smem > 48u * 1024u) {                        // held per device and context, so set where needed on each call
-            const int rc = cuda_status(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem),
+        if (smem > 48u * 1024u) {
+            // a limit, not an allocation, held per function and device: the same one on every call, so that calls on
+            // other threads never lower it ahead of this launch
+            const int rc = cuda_status(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kGridSmem),
                                        "grid shared memory");
             if (rc) return rc;
         }
@@ -560,7 +565,7 @@ int launch_grid_pa(const void* scene, int64_t n_atoms, int n_dirs, uint64_t seed
     // 124 / 81; on the line's other side 20,000 on 512: 91 / 114 and 239 / 335, 650 on 256: 27 / 36 and 36 / 42.
     if ((long long)n * n * n < 4096ll * n_atoms) {
         int rows = n;
-        while (rows > 1 && 4ll * rows * pitch > 136ll * 1024) rows /= 2;
+        while (rows > 1 && 4ll * rows * pitch > 136ll * 1024) rows /= 2;      // at most kGridSmem: a row is 1 KB
         const int bands = n / rows;
         // CTAs that share a direction's atoms: up to two an SM, 128 atoms each (20,000 atoms, one direction, 256 grid:
         // 527 us with one, 69 with eight)
@@ -577,7 +582,7 @@ int launch_grid_pa(const void* scene, int64_t n_atoms, int n_dirs, uint64_t seed
         return (unsigned)(kStage * (sizeof(float4) + sizeof(int2) + sizeof(short2) + 4) + 4 + warps * (kStage * 2 + 4 * words + 128 * pitch));
     };
     int warps = groups < 16 ? groups : 16;
-    while (warps > 2 && (bytes(warps) > 160u * 1024u || 5ll * n_dirs * (groups / warps) < sm_count())) warps /= 2;
+    while (warps > 2 && (bytes(warps) > (unsigned)kGridSmem || 5ll * n_dirs * (groups / warps) < sm_count())) warps /= 2;
     const int bands = groups / warps;
     while (parts < 8 && n_atoms > 256ll * parts && 2ll * n_dirs * bands * parts <= sm_count()) parts *= 2;
     return launch(k_grid_cover, bands, parts, 32 * warps, bytes(warps), words, pitch);

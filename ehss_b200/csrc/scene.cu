@@ -1431,14 +1431,16 @@ template <int THREADS, int ITEMS>
 static int launch_small(int S, int64_t max_n, int ctas, const BuildWork& W, const uint8_t* culled, cudaStream_t stream) {
     using B = SmallBuild<THREADS, ITEMS>;
     constexpr int kSmemPerSM = 227 * 1024, kStatic = 16 * 1024;     // scene_stats' static arrays, rounded up
+    static_assert(sizeof(B) + kStatic <= kSmemPerSM, "one CTA fits an SM");
     int boxes = (int)max_n - 1;
     if ((int64_t)(B::bytes(boxes) + kStatic) * ctas > kSmemPerSM) boxes = 0;
-    const int smem = (int)B::bytes(boxes);
-    // held per device and context, so set on each call (a limit, not an allocation)
+    // A limit, not an allocation, held per function and device: every call sets the same one, the largest that any call
+    // can need, so that calls on other threads never lower it ahead of this launch.
+    const int most = (int)std::min<int64_t>(B::bytes(B::kMax - 1), kSmemPerSM - kStatic);
     const int rc = cuda_status(cudaFuncSetAttribute(k_build_small<THREADS, ITEMS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                    smem), "LBVH build");
+                                                    most), "LBVH build");
     if (rc) return rc;
-    k_build_small<THREADS, ITEMS><<<S, THREADS, smem, stream>>>(W.descs, W.atom_scene, culled, W.inner_child, W.inner_range,
+    k_build_small<THREADS, ITEMS><<<S, THREADS, B::bytes(boxes), stream>>>(W.descs, W.atom_scene, culled, W.inner_child, W.inner_range,
                                                                 W.inner_box, W.leaf_box, W.inner_height, W.vals_out, boxes);
     return cuda_status(cudaGetLastError(), "LBVH build launch");
 }
