@@ -94,26 +94,39 @@ __device__ __forceinline__ float ray_ep(const SceneHeader* H) { return kEp * __l
 
 constexpr int kRayFar = 0, kRayOk = 1, kRayNotUnit = 2;
 
+// |d|^2 off by at most this counts as unit.  Other directions take the walk from
+// kShortest to kLongest of |d|^2, where the entry formula's margins, which are in
+// units of |d|, stay far below the filter's.
+constexpr double kUnitError = 1e-11, kShortest = 0x1p-40, kLongest = 0x1p40;
+
 // FP32 copy of an FP64 ray.  kRayFar: the origin is beyond 3 S from the centre
-// (or not finite), where node boxes are not widened enough.  kRayNotUnit: the
-// direction is off by more than 1e-11 in |d|^2, which the sphere test's
-// identity does not allow (boxes still hold: o is then the ray's own origin, and
-// distances along the ray are in units of |d|, so none is taken off them: Ep in
-// such units exceeds the boxes' widening from |d| = 20 on).  UNIT: the caller's
-// directions are unit to rounding.
-template <bool UNIT = false>
+// (or not finite), where node boxes are not widened enough.
+// Directions that are not unit (UNIT: there are none, the caller's are unit to
+// rounding): FILTER classifies along the normalised ray, whose spheres and order
+// of entries are the same, and FP64 decides with the caller's direction.  For
+// EXACT the boxes hold as they are, with o the ray's own origin and distances in
+// units of |d|, so none is taken off them (Ep in such units exceeds the boxes'
+// widening from |d| = 20 on); the sphere test's identity does not hold.
+// kRayNotUnit: such a ray, or one outside the range above.
+template <bool EXACT, bool UNIT>
 __device__ __forceinline__ int setup_ray(const SceneHeader* H, const double* o, const double* d, RayF& r) {
     const double x = o[0] - H->center[0], y = o[1] - H->center[1], z = o[2] - H->center[2];
     const float S = H->scale_f;
     const float fx = (float)x, fy = (float)y, fz = (float)z;
     if (!(sqrtf(fmaf(fx, fx, fmaf(fy, fy, fz * fz))) <= 3.0f * S)) return kRayFar;
     const double aa = fma(d[0], d[0], fma(d[1], d[1], d[2] * d[2]));
-    const bool unit = fabs(aa - 1.0) <= 1e-11;
-    const double tau0 = unit ? fma(x, d[0], fma(y, d[1], z * d[2])) : 0.0;
-    r.ox = (float)fma(-tau0, d[0], x);
-    r.oy = (float)fma(-tau0, d[1], y);
-    r.oz = (float)fma(-tau0, d[2], z);
-    const float dx = (float)d[0], dy = (float)d[1], dz = (float)d[2];
+    bool unit = fabs(aa - 1.0) <= kUnitError;
+    double d0 = d[0], d1 = d[1], d2 = d[2];
+    if (!EXACT && !UNIT && !unit && aa >= kShortest && aa <= kLongest) {
+        const double inv = 1.0 / sqrt(aa);
+        d0 *= inv; d1 *= inv; d2 *= inv;
+        unit = true;
+    }
+    const double tau0 = unit ? fma(x, d0, fma(y, d1, z * d2)) : 0.0;
+    r.ox = (float)fma(-tau0, d0, x);
+    r.oy = (float)fma(-tau0, d1, y);
+    r.oz = (float)fma(-tau0, d2, z);
+    const float dx = (float)d0, dy = (float)d1, dz = (float)d2;
     r.ix = safe_rcp(dx); r.iy = safe_rcp(dy); r.iz = safe_rcp(dz);
     r.dx = dx * kHalfSqrt2; r.dy = dy * kHalfSqrt2; r.dz = dz * kHalfSqrt2;
     const float q = fmaf(r.ox, r.ox, fmaf(r.oy, r.oy, r.oz * r.oz));
@@ -165,11 +178,13 @@ __device__ __forceinline__ float min3f(float a, float b, float c) {
 // misses without a check of its reference.  oi = o * inv + tau0 per axis
 // (distances from the ray's start), formed once per node visit (held per lane
 // it would cost three registers of the fused kernel).
+template <bool WIDE>
 __device__ __forceinline__ float box_enter(const RayF& r, float oix, float oiy, float oiz, float nx, float fx, float ny,
-                                           float fy, float nz, float fz, float U) {
+                                           float fy, float nz, float fz, float U, float wx, float wy, float wz) {
     float tnx = fmaf(nx, r.ix, -oix), tfx = fmaf(fx, r.ix, -oix);
     float tny = fmaf(ny, r.iy, -oiy), tfy = fmaf(fy, r.iy, -oiy);
     float tnz = fmaf(nz, r.iz, -oiz), tfz = fmaf(fz, r.iz, -oiz);
+    if (WIDE) { tnx -= wx; tfx += wx; tny -= wy; tfy += wy; tnz -= wz; tfz += wz; }
     float tmin = max3f(tnx, tny, fmaxf(tnz, 0.0f));
     float tmax = min3f(tfx, tfy, fminf(tfz, U));
     return tmin <= tmax ? tmin : CUDART_INF_F;
@@ -190,7 +205,10 @@ __device__ __forceinline__ void cswap(Hits4& h, int a, int b) {
     h.t[a] = ta; h.t[b] = tb; h.ref[a] = ra; h.ref[b] = rb;
 }
 
-__device__ __forceinline__ Hits4 visit4(const float4* nodes, int node, const RayF& r, float U) {
+// WIDE: the planes of axis x (y, z) are moved wx (wy, wz) along the ray apart.
+template <bool WIDE = false>
+__device__ __forceinline__ Hits4 visit4(const float4* nodes, int node, const RayF& r, float U, float wx = 0.f, float wy = 0.f,
+                                        float wz = 0.f) {
     const float4* nd = nodes + 8 * (int64_t)node;
     // near and far plane rows by the direction's sign per axis (the node stores lo, hi)
     const int sx = __float_as_uint(r.ix) >> 31, sy = __float_as_uint(r.iy) >> 31, sz = __float_as_uint(r.iz) >> 31;
@@ -202,10 +220,10 @@ __device__ __forceinline__ Hits4 visit4(const float4* nodes, int node, const Ray
     // distances from the ray's start (less Ep, which the boxes' widening absorbs)
     const float tau0 = r.bmin * kSqrt2;
     const float oix = fmaf(r.ox, r.ix, tau0), oiy = fmaf(r.oy, r.iy, tau0), oiz = fmaf(r.oz, r.iz, tau0);
-    h.t[0] = box_enter(r, oix, oiy, oiz, nx.x, fx.x, ny.x, fy.x, nz.x, fz.x, U);
-    h.t[1] = box_enter(r, oix, oiy, oiz, nx.y, fx.y, ny.y, fy.y, nz.y, fz.y, U);
-    h.t[2] = box_enter(r, oix, oiy, oiz, nx.z, fx.z, ny.z, fy.z, nz.z, fz.z, U);
-    h.t[3] = box_enter(r, oix, oiy, oiz, nx.w, fx.w, ny.w, fy.w, nz.w, fz.w, U);
+    h.t[0] = box_enter<WIDE>(r, oix, oiy, oiz, nx.x, fx.x, ny.x, fy.x, nz.x, fz.x, U, wx, wy, wz);
+    h.t[1] = box_enter<WIDE>(r, oix, oiy, oiz, nx.y, fx.y, ny.y, fy.y, nz.y, fz.y, U, wx, wy, wz);
+    h.t[2] = box_enter<WIDE>(r, oix, oiy, oiz, nx.z, fx.z, ny.z, fy.z, nz.z, fz.z, U, wx, wy, wz);
+    h.t[3] = box_enter<WIDE>(r, oix, oiy, oiz, nx.w, fx.w, ny.w, fy.w, nz.w, fz.w, U, wx, wy, wz);
     cswap(h, 0, 1); cswap(h, 2, 3); cswap(h, 0, 2); cswap(h, 1, 3); cswap(h, 1, 2);
     h.n = (h.t[0] != CUDART_INF_F) + (h.t[1] != CUDART_INF_F) + (h.t[2] != CUDART_INF_F) + (h.t[3] != CUDART_INF_F);
     return h;
@@ -243,7 +261,7 @@ __device__ __forceinline__ int nearest(const SceneView& S, const double* o, cons
                                     double& best_out, LocalStats& st) {
     ++st.queries;
     RayF r;
-    const int kind = setup_ray<UNIT>(S.h, o, d, r);
+    const int kind = setup_ray<EXACT, UNIT>(S.h, o, d, r);
     if (kind == kRayFar) return nearest_flat(S, o, d, last_rank, best_out, st);
     if (!EXACT && kind == kRayNotUnit) { --st.queries; return nearest<true, UNIT>(S, o, d, last_rank, best_out, st); }
     const float Edisc = ray_edisc(S.h), Ep = ray_ep(S.h);
@@ -364,23 +382,23 @@ __device__ __noinline__ int nearest_call(const SceneView& S, const double* o, co
     return nearest<EXACT>(S, o, d, last_rank, best_out, st);
 }
 
-// Any-hit PA query (pa_spatial._one with sphere_hit): true when the ray
-// meets any sphere other than owner_rank.
-__device__ __noinline__ bool anyhit(const SceneView& S, const double* o, const double* d, int owner_rank,
-                                    LocalStats& st) {
-    ++st.queries;
-    RayF r;
-    if (setup_ray(S.h, o, d, r) != kRayOk) {
-        int n = S.h->n_atoms;
-        for (int k = 0; k < n; ++k) {
-            if (k == owner_rank) continue;
-            double4 a = S.atoms64[k];
-            ++st.sphere; ++st.fp64;
-            if (sphere_hit64(o[0], o[1], o[2], d[0], d[1], d[2], a.x, a.y, a.z, a.w)) return true;
-        }
-        return false;
-    }
+// Direction off unit length, for the any-hit query: sphere_hit takes |d| = 1, so
+// with e = |d|^2 - 1 and b the distance along the line of its point nearest the
+// centre, its discriminant is the normalised ray's plus e b^2, |b| <= |o| + S.
+// Certain misses and hits keep that much more distance (more, less), and boxes
+// are moved sqrt(more) apart, at most 8 S, where every box holds the origin: the
+// ray meets nothing farther than that from a sphere.
+struct OffUnit {
+    float more, less, wx, wy, wz;
+};
+
+// Any-hit walk (pa_spatial._one with sphere_hit): true when the ray meets any
+// sphere other than owner_rank.
+template <bool UNIT>
+__device__ __forceinline__ bool anyhit_walk(const SceneView& S, const RayF& r, const double* o, const double* d, int owner_rank,
+                                            const OffUnit& f, LocalStats& st) {
     const float Edisc = ray_edisc(S.h), Ep = ray_ep(S.h);
+    const float miss = UNIT ? r.thr : r.thr - 0.5f * f.more, hit = UNIT ? 2.0f * Edisc : fmaf(2.0f, Edisc, f.less);
     int stack_ref[kStackDepth];
     int sp = 0;
     int cur = 0;
@@ -389,7 +407,7 @@ __device__ __noinline__ bool anyhit(const SceneView& S, const double* o, const d
     for (int steps = 0;; ++steps) {
         if (cur >= n_nodes || steps > 2 * n_nodes + 2) { ++st.errors; break; }
         if (cur >= 0) {
-            Hits4 h = visit4(S.nodes, cur, r, U);
+            Hits4 h = visit4<!UNIT>(S.nodes, cur, r, U, f.wx, f.wy, f.wz);
             st.box += 4;
             if (h.n > 0) {
                 for (int k = h.n - 1; k >= 1; --k) {
@@ -408,9 +426,9 @@ __device__ __noinline__ bool anyhit(const SceneView& S, const double* o, const d
                 const float4 a = __ldg(S.atoms + k);
                 float b;
                 const float D = sphere_disc(r, a, b);
-                if (D < r.thr) continue;
+                if (D < miss) continue;
                 const float disc = fmaf(2.0f, D - r.thr, -Edisc), bt = fmaf(b - r.bmin, kSqrt2, -Ep);
-                if (disc >= 2.0f * Edisc) {
+                if (disc >= hit) {
                     float Et;
                     // far root: the reference's -b + sqrt(disc) with b = x.d = -(v.d)
                     const float exitp = bt + certain_sqrt(bt, disc, Ep, Edisc, Et);
@@ -426,6 +444,40 @@ __device__ __noinline__ bool anyhit(const SceneView& S, const double* o, const d
         }
         if (sp == 0) break;
         cur = stack_ref[--sp];
+    }
+    return false;
+}
+
+// Any-hit PA query of a ray.  UNIT: the caller's directions are unit to rounding.
+template <bool UNIT>
+__device__ __noinline__ bool anyhit(const SceneView& S, const double* o, const double* d, int owner_rank,
+                                    LocalStats& st) {
+    ++st.queries;
+    RayF r;
+    if (setup_ray<false, UNIT>(S.h, o, d, r) == kRayOk) {
+        OffUnit f = {0.f, 0.f, 0.f, 0.f, 0.f};
+        if (UNIT) return anyhit_walk<true>(S, r, o, d, owner_rank, f, st);
+        const double e = fma(d[0], d[0], fma(d[1], d[1], d[2] * d[2])) - 1.0;
+        if (fabs(e) > kUnitError) {
+            const float scale = S.h->scale_f;
+            const double x = o[0] - S.h->center[0], y = o[1] - S.h->center[1], z = o[2] - S.h->center[2];
+            const float reach = sqrtf((float)fma(x, x, fma(y, y, z * z))) + scale, change = 1.001f * (float)fabs(e) * reach * reach;
+            // lines beyond S meet such spheres too: the bound of the FP32 test for |o| up to 3 S, 72u S^2, takes 24u more
+            const float error = 32.0f * kU32 * scale * scale;
+            r.thr = 0.5f * (fmaf(r.ox, r.ox, fmaf(r.oy, r.oy, r.oz * r.oz)) - kEdisc * scale * scale);
+            f.more = e > 0.0 ? change + error : error;
+            f.less = e > 0.0 ? error : change + error;
+            const float wide = fminf(1.001f * sqrtf(f.more), 8.0f * scale);
+            f.wx = wide * fabsf(r.ix); f.wy = wide * fabsf(r.iy); f.wz = wide * fabsf(r.iz);
+        }
+        return anyhit_walk<false>(S, r, o, d, owner_rank, f, st);
+    }
+    const int n = S.h->n_atoms;
+    for (int k = 0; k < n; ++k) {
+        if (k == owner_rank) continue;
+        const double4 a = S.atoms64[k];
+        ++st.sphere; ++st.fp64;
+        if (sphere_hit64(o[0], o[1], o[2], d[0], d[1], d[2], a.x, a.y, a.z, a.w)) return true;
     }
     return false;
 }
@@ -487,7 +539,7 @@ __global__ void __launch_bounds__(128) k_pa_rays(const void* scene, int64_t n, c
         if (i >= n) continue;
         int64_t owner = owners ? owners[i] : -1;
         if (!ok || owner < -1 || owner >= S.h->n_atoms) { ++st.errors; blocked[i] = 0; continue; }
-        blocked[i] = anyhit(S, o, d, owner >= 0 ? S.rank[owner] : -1, st);
+        blocked[i] = anyhit<false>(S, o, d, owner >= 0 ? S.rank[owner] : -1, st);
     }
     __syncwarp();
     flush_stats(st, stats);
@@ -756,7 +808,7 @@ struct Walker {
     // for FILTER a direction that is not unit).
     __device__ __forceinline__ int start(const SceneHeader* H, const LaneRay& L) {
         reset();
-        const int kind = setup_ray<UNIT>(H, L.o, L.d, r);
+        const int kind = setup_ray<EXACT, UNIT>(H, L.o, L.d, r);
         if (!EXACT || kind == kRayFar) return kind;
         r.thr = kind == kRayOk ? 0.0f : CUDART_INF_F;
         return kRayOk;
@@ -915,7 +967,7 @@ __global__ void __launch_bounds__(128, 8) k_blocks(const ehss_block* blocks, int
                 (__ldg(&B->flags) & EHSS_BLOCK_PA)) {
                 // a near-tangent first query leaves PA (below) to the any-hit query
                 LocalStats pst;
-                if (anyhit(scene_view(sbase), L.o, L.d, -1, pst)) atomicAdd(&A.pa, 1u);
+                if (anyhit<!RAYS>(scene_view(sbase), L.o, L.d, -1, pst)) atomicAdd(&A.pa, 1u);
                 if (COUNT) { W.box += pst.box; W.sphere += pst.sphere; }
             }
             if (!EXACT && status == kDone && W.overflow && !W.error) {
@@ -1008,7 +1060,7 @@ __global__ void __launch_bounds__(128, 8) k_blocks(const ehss_block* blocks, int
                         }
                         if (PA && (__ldg(&B->flags) & EHSS_BLOCK_PA) && (RAYS || !(__ldg(&B->flags) & EHSS_BLOCK_EHSS))) {
                             LocalStats pst;
-                            if (anyhit(S, L.o, L.d, -1, pst)) {
+                            if (anyhit<!RAYS>(S, L.o, L.d, -1, pst)) {
                                 atomicAdd(&A.pa, 1u);
                                 if (RAYS) atomicAdd(&A.pa_fx, __double2ull_rn(*rho_lane * kFxScale));
                             }
