@@ -742,9 +742,11 @@ def main():
     if rank == 0 and world == 1 and not args.no_serve:
         serve = serving_measurement()
     if rank == 0:
-        # builder: two passes of one tree kernel (one CTA a structure: every structure here holds at
-        # most 8192 atoms) and the emission, the exposure test between them; then 1 persistent trace kernel
-        launches_per_step = 2 * 2 + 1 + 1
+        # builder: two passes around the exposure test, every structure here holding at most 8192 atoms;
+        # more than 8 structures: scene index + stats, 5 tree kernels a pass (keys sorted per structure in
+        # one kernel), a fix-up behind the exposure test; up to 8: one tree kernel (one CTA a structure) and
+        # two emission kernels a pass.  Then 1 persistent trace kernel
+        launches_per_step = (2 + 5 * 2 + 2 if len(structures) > 8 else 3 * 2 + 1) + 1
         line = {"metric": METRIC, "value": value, "unit": UNIT, "n_gpus": world, "steps": args.steps,
                 "warmup": args.warmup, "ms_per_step": total_ms / args.steps, "higher_is_better": True,
                 "scaling": "weak", "vs_baseline": None, "dtype": "f32+f64", "data": "synthetic",

@@ -17,6 +17,8 @@
 //                  structure's centre box; key = structure << 31 | buried << 30
 //                  | code (buried only in the second pass of an exterior build)
 //   3. stable sort of (key, atom) pairs, so equal codes keep atom order:
+//                  per structure in one CTA (k_morton_segsort, steps 2-3 in one
+//                  launch) when every structure holds at most 8192 atoms, else
 //                  a device-wide LSD radix sort over the key's significant bits
 //                  (k_radix_count / k_radix_scan / k_radix_scatter, 8 bits a pass)
 //   4. k_karras    per internal node: Karras (2012) range / split search
@@ -28,8 +30,8 @@
 //                  by eps_box; subtrees of at most leaf_size atoms collapsed
 //                  into leaf references); per atom: FP32 and FP64 records in
 //                  leaf order, id maps.
-// Batches of structures of at most 8192 atoms run all of it in one launch,
-// one CTA a structure (k_build_small).
+// Up to 8 structures of at most 8192 atoms: steps 1-5 in one launch, one CTA a
+// structure (k_build_small).
 // Exterior builds (EHSS_BUILD_EXTERIOR) then run k_exposure on that tree and
 // repeat steps 2-6 with the buried atoms sorted behind the exposed ones and
 // left out of the tree.
@@ -276,7 +278,43 @@ __global__ void k_morton(const BuildDesc* descs, const int32_t* atom_scene, int6
     vals[g] = (int32_t)i;
 }
 
-constexpr int kSegSortMax = 8192;      // batches of structures up to here build with one CTA each (k_build_small)
+// Batches whose structures all hold at most kSegSortMax atoms: keys made and
+// sorted per structure by one CTA (stable block radix sort in shared memory),
+// one launch instead of the device-wide sort's several.  Keys never cross
+// structures, so the result equals the device-wide stable sort of k_morton's
+// keys element for element.  Two sizes: 256 x 8 keys (structures of at most
+// 2048 atoms) and 512 x 16 (8192).
+constexpr int kSegSortMax = 8192, kSegSortSmall = 2048;
+
+template <int THREADS, int ITEMS>
+__global__ void __launch_bounds__(THREADS, 1024 / THREADS) k_morton_segsort(const BuildDesc* descs,
+                                                                          const uint8_t* culled,
+                                                                          uint64_t* keys_out, int32_t* vals_out) {
+    using SegSort = cub::BlockRadixSort<uint32_t, THREADS, ITEMS, int32_t>;
+    static_assert(sizeof(typename SegSort::TempStorage) <= 48 * 1024, "segment sort storage fits static shared memory");
+    __shared__ typename SegSort::TempStorage temp;
+    const int s = blockIdx.x;
+    const BuildDesc& D = descs[s];
+    const SceneHeader* H = reinterpret_cast<const SceneHeader*>(D.scene);
+    const int n = D.n < THREADS * ITEMS ? (int)D.n : THREADS * ITEMS;     // the host sends no larger structure
+    uint32_t key[ITEMS];
+    int32_t val[ITEMS];
+#pragma unroll
+    for (int k = 0; k < ITEMS; ++k) {
+        const int i = threadIdx.x * ITEMS + k;              // blocked: item order = atom order
+        val[k] = i;
+        key[k] = i < n ? morton_key31(D, H, i, culled && D.exterior && culled[D.atom0 + i]) : 0xffffffffu;
+    }
+    SegSort(temp).Sort(key, val, 0, 32);
+#pragma unroll
+    for (int k = 0; k < ITEMS; ++k) {
+        const int j = threadIdx.x * ITEMS + k;
+        if (j < n) {
+            keys_out[D.atom0 + j] = ((uint64_t)s << 31) | key[k];
+            vals_out[D.atom0 + j] = val[k];
+        }
+    }
+}
 
 // --------------------------------------------------------------------------
 // Device-wide stable LSD radix sort of (uint64 key, int32 value) pairs, for
@@ -621,38 +659,37 @@ __device__ __forceinline__ void emit_atom(const BuildDesc& D, const SceneHeader*
     rank[a] = (int32_t)j;
 }
 
-// All records of a batch: threads 0 .. N-1 the atoms, then the internal nodes,
-// then one a structure for its header.
-__global__ void k_emit(const BuildDesc* descs, int n_scenes, const int32_t* atom_scene, int64_t N, int64_t I_total,
-                       const int32_t* vals_sorted, const int32_t* inner_child, const int32_t* inner_range,
-                       const float* inner_box, const float* leaf_box, const int32_t* inner_height) {
-    int64_t g = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (g < N) {
-        const BuildDesc& D = descs[atom_scene[g]];
-        emit_atom(D, reinterpret_cast<const SceneHeader*>(D.scene), g - D.atom0, vals_sorted[g]);
+// Node records of a batch, and one more thread a structure for its header.
+__global__ void k_emit_nodes(const BuildDesc* descs, int n_scenes, int64_t I_total, const int32_t* inner_child,
+                             const int32_t* inner_range, const float* inner_box, const float* leaf_box,
+                             const int32_t* inner_height) {
+    const int64_t g = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    if (g >= I_total + n_scenes) return;
+    if (g >= I_total) {
+        const BuildDesc& D = descs[g - I_total];
+        finish_header(D, reinterpret_cast<SceneHeader*>(D.scene), leaf_box + 6 * D.atom0,
+                      D.n_active > 1 ? inner_height[D.inner0] : 0);
         return;
     }
-    g -= N;
-    if (g < I_total) {
-        const BuildDesc& D = descs[node_owner(descs, n_scenes, g)];
-        const int i = (int)(g - D.inner0);
-        if (i >= D.n_active - 1 || D.n_active <= D.leaf_size) return;
-        emit_node(D, reinterpret_cast<const SceneHeader*>(D.scene), i, inner_child + 2 * D.inner0, inner_range + 2 * D.inner0,
-                  inner_box + 6 * D.inner0, leaf_box + 6 * D.atom0);
-        return;
-    }
-    g -= I_total;
-    if (g >= n_scenes) return;
-    const BuildDesc& D = descs[g];
-    finish_header(D, reinterpret_cast<SceneHeader*>(D.scene), leaf_box + 6 * D.atom0,
-                  D.n_active > 1 ? inner_height[D.inner0] : 0);
+    const BuildDesc& D = descs[node_owner(descs, n_scenes, g)];
+    const int i = (int)(g - D.inner0);
+    if (i >= D.n_active - 1 || D.n_active <= D.leaf_size) return;
+    emit_node(D, reinterpret_cast<const SceneHeader*>(D.scene), i, inner_child + 2 * D.inner0, inner_range + 2 * D.inner0,
+              inner_box + 6 * D.inner0, leaf_box + 6 * D.atom0);
+}
+
+__global__ void k_emit_atoms(const BuildDesc* descs, const int32_t* atom_scene, int64_t N, const int32_t* vals_sorted) {
+    const int64_t g = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    if (g >= N) return;
+    const BuildDesc& D = descs[atom_scene[g]];
+    emit_atom(D, reinterpret_cast<const SceneHeader*>(D.scene), g - D.atom0, vals_sorted[g]);
 }
 
 // --------------------------------------------------------------------------
-// Batches whose structures all hold at most kSegSortMax atoms: one CTA makes
+// Up to kOneCtaTrees structures, all of at most kSegSortMax atoms: one CTA makes
 // one structure's tree in one launch (a launch a pass: the full tree, and for
-// exterior scenes the tree over the exposed atoms after k_exposure), and k_emit
-// writes the records on all SMs.  The phases are those of the device-wide path
+// exterior scenes the tree over the exposed atoms after k_exposure), and
+// k_emit_nodes and k_emit_atoms write the records on all SMs.  The phases are those of the device-wide path
 // -- statistics, Morton keys and their stable sort, Karras hierarchy, bottom-up
 // boxes -- with __syncthreads between them instead of launches; the sorted
 // keys, parent links, arrival flags and (where they fit) the node boxes lie in
@@ -661,9 +698,7 @@ __global__ void k_emit(const BuildDesc* descs, int n_scenes, const int32_t* atom
 // device-wide path's byte for byte.
 // Bound by latency: of the full tree of 5000 atoms (160 us) the sequential
 // coordinate sum takes 30 % (none where the caller gives the centre), the sort
-// 25 %, the walk up 35 %.  Both passes with
-// k_emit: 72 us for 650 atoms (160 us as eleven launches), 163 us for 5000
-// (260), 355 us for 256 structures of 20-5000 atoms (435).
+// 25 %, the walk up 35 %.
 // THREADS x ITEMS is the largest structure of the instance; smaller ones sort
 // with half or a quarter of the items, as they are.
 // --------------------------------------------------------------------------
@@ -687,6 +722,12 @@ struct SmallBuild {
     uint32_t key[kMax];                // then, from here on, the node boxes if the launch has room for them
     static size_t bytes(int64_t boxes) { return sizeof(SmallBuild) - sizeof(key) + std::max(sizeof(key), 24 * (size_t)boxes); }
 };
+// Most structures of a batch that are built this way; more take the passes above, a launch each.  Exterior build of
+// one, 8, 16 and 256 structures, passes / one CTA in us: 650 atoms 200 / 115, 249 / 150, 278 / 175, 1103 / 981; 20 to
+// 5000 atoms 343 / 320, 367 / 338, 408 / 377, 1765 / 1696.  One CTA is the faster on both sides of the line: where the
+// launches are what a build costs, by up to 1.7 times; in a batch by 4 to 9 % of a build that is a tenth of the step.
+// Batches keep the 15 launches a step that bench.py states and its test expects.
+constexpr int kOneCtaTrees = 8;
 constexpr int kNoParent = 0xffff;
 constexpr unsigned kNobody = 0xffffffffu, kIsLeaf = 0x80000000u;
 
@@ -1426,32 +1467,30 @@ uint64_t build_workspace_bytes(int64_t N, int S) {
 }
 
 // k_build_small, the instance for structures of at most max_n atoms.  Node
-// boxes go to shared memory where an SM holds `ctas` such CTAs.
+// boxes go to shared memory where an SM has room for them.
 template <int THREADS, int ITEMS>
-static int launch_small(int S, int64_t max_n, int ctas, const BuildWork& W, const uint8_t* culled, cudaStream_t stream) {
+static int launch_small(int S, int64_t max_n, const BuildWork& W, const uint8_t* culled, cudaStream_t stream) {
     using B = SmallBuild<THREADS, ITEMS>;
     constexpr int kSmemPerSM = 227 * 1024, kStatic = 16 * 1024;     // scene_stats' static arrays, rounded up
     static_assert(sizeof(B) + kStatic <= kSmemPerSM, "one CTA fits an SM");
     int boxes = (int)max_n - 1;
-    if ((int64_t)(B::bytes(boxes) + kStatic) * ctas > kSmemPerSM) boxes = 0;
+    if ((int64_t)B::bytes(boxes) + kStatic > kSmemPerSM) boxes = 0;
     // A limit, not an allocation, held per function and device: every call sets the same one, the largest that any call
     // can need, so that calls on other threads never lower it ahead of this launch.
     const int most = (int)std::min<int64_t>(B::bytes(B::kMax - 1), kSmemPerSM - kStatic);
     const int rc = cuda_status(cudaFuncSetAttribute(k_build_small<THREADS, ITEMS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                                     most), "LBVH build");
     if (rc) return rc;
-    k_build_small<THREADS, ITEMS><<<S, THREADS, B::bytes(boxes), stream>>>(W.descs, W.atom_scene, culled, W.inner_child, W.inner_range,
-                                                                W.inner_box, W.leaf_box, W.inner_height, W.vals_out, boxes);
+    k_build_small<THREADS, ITEMS><<<S, THREADS, B::bytes(boxes), stream>>>(W.descs, W.atom_scene, culled, W.inner_child,
+                                                                           W.inner_range, W.inner_box, W.leaf_box,
+                                                                           W.inner_height, W.vals_out, boxes);
     return cuda_status(cudaGetLastError(), "LBVH build launch");
 }
 
 static int launch_build_small(int S, int64_t max_n, const BuildWork& W, const uint8_t* culled, cudaStream_t stream) {
-    // one CTA an SM while every structure has an SM to itself, else two
-    const bool few = S <= sm_count();
-    if (max_n <= 1024) return launch_small<512, 2>(S, max_n, few ? 1 : 3, W, culled, stream);
-    if (max_n <= 2048) return few ? launch_small<1024, 2>(S, max_n, 1, W, culled, stream)
-                                  : launch_small<512, 4>(S, max_n, 2, W, culled, stream);
-    return few ? launch_small<1024, 8>(S, max_n, 1, W, culled, stream) : launch_small<512, 16>(S, max_n, 2, W, culled, stream);
+    if (max_n <= 1024) return launch_small<512, 2>(S, max_n, W, culled, stream);
+    if (max_n <= 2048) return launch_small<1024, 2>(S, max_n, W, culled, stream);
+    return launch_small<1024, 8>(S, max_n, W, culled, stream);
 }
 
 int build_scenes(int S, const double* const* xyz, const double* const* radii, const int64_t* n, int leaf_size,
@@ -1534,7 +1573,7 @@ int build_scenes(int S, const double* const* xyz, const double* const* radii, co
 
     const int T = 256;
     auto blocks = [&](int64_t count) { return (unsigned)((count + T - 1) / T); };
-    const bool small = max_n <= kSegSortMax;
+    const bool segsort = max_n <= kSegSortMax, small = segsort && S <= kOneCtaTrees;
     if (!small) {
         k_fill_scene_index<<<S, 256, 0, stream>>>(W.descs, S, W.atom_scene);
         k_stats<<<S, 256, 0, stream>>>(W.descs, S);
@@ -1548,28 +1587,37 @@ int build_scenes(int S, const double* const* xyz, const double* const* radii, co
             r = launch_build_small(S, max_n, W, culled, stream);
             if (r) return r;
         } else {
-        // the keys start in the buffer from which an odd or even number of passes ends in keys_out
-        const bool odd = radix_passes(end_bit) % 2 != 0;
-        k_morton<<<blocks(N), T, 0, stream>>>(W.descs, W.atom_scene, N, culled, odd ? W.keys_in : W.keys_out,
-                                              odd ? W.vals_in : W.vals_out);
-        r = radix_sort_pairs(W.keys_in, W.vals_in, W.keys_out, W.vals_out, N, end_bit, W.radix_counts,
-                             W.radix_offsets, stream);
-        if (r) return r;
-        // parent links start at -1 so that a missing link ends a refit walk
-        r = cuda_status(cudaMemsetAsync(W.parent_leaf, 0xff, 4ull * N, stream), "LBVH parent reset");
-        if (r) return r;
-        if (I > 0) {
-            r = cuda_status(cudaMemsetAsync(W.arrivals, 0, 4ull * I, stream), "LBVH arrival reset");
-            if (!r) r = cuda_status(cudaMemsetAsync(W.parent_inner, 0xff, 4ull * I, stream), "LBVH parent reset");
+            if (segsort) {
+                if (max_n <= kSegSortSmall)
+                    k_morton_segsort<256, 8><<<S, 256, 0, stream>>>(W.descs, culled, W.keys_out, W.vals_out);
+                else
+                    k_morton_segsort<512, 16><<<S, 512, 0, stream>>>(W.descs, culled, W.keys_out, W.vals_out);
+                r = cuda_status(cudaGetLastError(), "LBVH key sort");
+            } else {
+                // the keys start in the buffer from which an odd or even number of passes ends in keys_out
+                const bool odd = radix_passes(end_bit) % 2 != 0;
+                k_morton<<<blocks(N), T, 0, stream>>>(W.descs, W.atom_scene, N, culled, odd ? W.keys_in : W.keys_out,
+                                                      odd ? W.vals_in : W.vals_out);
+                r = radix_sort_pairs(W.keys_in, W.vals_in, W.keys_out, W.vals_out, N, end_bit, W.radix_counts,
+                                     W.radix_offsets, stream);
+            }
             if (r) return r;
-            k_karras<<<blocks(I), T, 0, stream>>>(W.descs, S, I, W.keys_out, W.inner_child, W.inner_range,
-                                                  W.parent_inner, W.parent_leaf);
+            // parent links start at -1 so that a missing link ends a refit walk
+            r = cuda_status(cudaMemsetAsync(W.parent_leaf, 0xff, 4ull * N, stream), "LBVH parent reset");
+            if (r) return r;
+            if (I > 0) {
+                r = cuda_status(cudaMemsetAsync(W.arrivals, 0, 4ull * I, stream), "LBVH arrival reset");
+                if (!r) r = cuda_status(cudaMemsetAsync(W.parent_inner, 0xff, 4ull * I, stream), "LBVH parent reset");
+                if (r) return r;
+                k_karras<<<blocks(I), T, 0, stream>>>(W.descs, S, I, W.keys_out, W.inner_child, W.inner_range,
+                                                      W.parent_inner, W.parent_leaf);
+            }
+            k_refit<<<blocks(N), T, 0, stream>>>(W.descs, W.atom_scene, N, W.vals_out, W.inner_child, W.parent_inner,
+                                                 W.parent_leaf, W.inner_box, W.leaf_box, W.inner_height, W.arrivals);
         }
-        k_refit<<<blocks(N), T, 0, stream>>>(W.descs, W.atom_scene, N, W.vals_out, W.inner_child, W.parent_inner,
-                                             W.parent_leaf, W.inner_box, W.leaf_box, W.inner_height, W.arrivals);
-        }
-        k_emit<<<blocks(N + I + S), T, 0, stream>>>(W.descs, S, W.atom_scene, N, I, W.vals_out, W.inner_child, W.inner_range,
-                                                    W.inner_box, W.leaf_box, W.inner_height);
+        k_emit_nodes<<<blocks(I + S), T, 0, stream>>>(W.descs, S, I, W.inner_child, W.inner_range, W.inner_box, W.leaf_box,
+                                                      W.inner_height);
+        k_emit_atoms<<<blocks(N), T, 0, stream>>>(W.descs, W.atom_scene, N, W.vals_out);
         return cuda_status(cudaGetLastError(), "LBVH build launch");
     };
     rc = tree_pass(nullptr);
