@@ -219,16 +219,23 @@ class DeviceExecutor:
         self.precision = {'fp64': _lib.PREC_FP64, 'fp32': _lib.PREC_FP32}[precision]
 
     def warmup(self, sizes=(64, 4096, 12000)):
-        """Build and trace one synthetic structure per builder path (per-structure
-        key sorts of up to 2048 and 8192 atoms, the device-wide sort above) so
-        that the first requests of each size do not wait for kernels to load."""
+        """Build and trace one synthetic structure of each size, then build by
+        the paths that those do not take (scene.cu: one CTA a structure in three
+        sizes, up to 1024, 2048 and 8192 atoms, for up to 8 structures; key sorts
+        a structure in two sizes for more; the device-wide sort above 8192 atoms),
+        so that the first requests do not wait for kernels to load."""
         rng = np.random.default_rng(0)
-        for n in sizes:
+
+        def synthetic(n):
             side = int(np.ceil(n ** (1. / 3.)))
             grid = np.stack(np.meshgrid(*[np.arange(side)] * 3, indexing='ij'), -1).reshape(-1, 3)[:n] * 2.5
-            structure = (grid + rng.normal(0., 0.05, grid.shape), np.full(n, 1.6))
-            handle = self.build([structure])[0]
+            return grid + rng.normal(0., 0.05, grid.shape), np.full(n, 1.6)
+        for n in sizes:
+            handle = self.build([synthetic(n)])[0]
             self.trace([(handle, 12, 1)])
+        for n, copies in ((64, 1), (1536, 1), (4096, 1), (64, 9), (2560, 9), (12000, 1)):
+            if copies > 1 or n not in sizes:
+                self.build([synthetic(n)] * copies)
 
     def footprint(self, n_atoms):
         """Device bytes one request may hold: its scene, its share of the
