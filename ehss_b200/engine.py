@@ -174,6 +174,23 @@ def _host_array(a, dtype):
     return np.require(a, dtype, ['C', 'A'])
 
 
+def _per_ray(a, dtype, shape):
+    """The entries of ``shape[0]`` rays, as _host_array: longer arrays are read
+    up to there, and one entry for all rays is repeated."""
+    a = np.asarray(a)
+    if a.shape != shape:
+        a = np.broadcast_to(a[:shape[0]], shape)
+    return _host_array(a, dtype)
+
+
+def _rows(a, dtype, n, width):
+    """The first n rows of ``width`` entries, as _host_array."""
+    a = _host_array(np.atleast_1d(a), dtype)
+    if len(a) < n or a.size != width * len(a):
+        raise ValueError('One origin, direction and owner per ray required')
+    return a.reshape(-1, width)[:n]
+
+
 def _reachable(a, device, hold):
     """Address of a contiguous host array that kernels can read where it lies
     (page-locked memory), or of a device copy; ``hold`` keeps it alive."""
@@ -218,10 +235,11 @@ class GPUEHSSTransport:
             raise ValueError('Positive cap and zero/one initial collision required')
         start = time.perf_counter()
         n = len(source.weights)
-        origins, directions = (_host_array(a, np.float64) for a in (source.origins, source.directions))
-        last, bounces = (_host_array(a, np.int64) for a in (source.last_atom, source.initial_bounces))
-        if origins.shape != (n, 3) or directions.shape != (n, 3) or last.shape != (n,) or bounces.shape != (n,):
-            raise ValueError('One origin, direction, initial identity and bounce count per weight required')
+        try:
+            origins, directions = (_per_ray(a, np.float64, (n, 3)) for a in (source.origins, source.directions))
+            last, bounces = (_per_ray(a, np.int64, (n,)) for a in (source.last_atom, source.initial_bounces))
+        except (ValueError, IndexError):
+            raise ValueError('One origin, direction, initial identity and bounce count per weight required') from None
         # A source starts without colliders (-1) and collisions as a rule.  Where its ends say so, the device traces
         # it that way while the host reads the two arrays through; if an entry differs, the result is dropped and
         # the arrays are checked and traced as they are.
@@ -345,11 +363,9 @@ class SphereIndex:
         owners = getattr(source, 'owners', None)
         if owners is None:
             owners = source.last_atom
-        origins, directions = (_host_array(a, np.float64) for a in (source.origins, source.directions))
-        own = _host_array(owners, np.int64)
-        n = len(origins)
-        if origins.shape != (n, 3) or directions.shape != (n, 3) or own.shape != (n,):
-            raise ValueError('One origin, direction and owner per ray required')
+        n = len(source.origins)
+        origins, directions = (_rows(a, np.float64, n, 3) for a in (source.origins, source.directions))
+        own = _rows(owners, np.int64, n, 1).reshape(-1)
         # rays without an owner (-1) are the rule: traced so while the host reads the owners through (as in trace)
         done = None
         if _ends_equal(own, -1):
