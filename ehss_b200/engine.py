@@ -171,7 +171,8 @@ def external_source(spheres, power, seed, scene=None):
 def _host_array(a, dtype):
     """``a`` as a C-contiguous array whose elements lie on their own alignment,
     as kernels need them: itself where it is one, else a copy."""
-    return np.require(a, dtype, ['C', 'A'])
+    a = np.ascontiguousarray(a, dtype=dtype)
+    return a if a.flags.aligned else a.copy()
 
 
 def _per_ray(a, dtype, shape):
@@ -207,11 +208,42 @@ def _page_locked(device, sizes):
         starts.append(total)
         total += -(-n // 64) * 64
     buf = torch().empty(max(total, 1), dtype=torch().uint8, pin_memory=True)
-    return buf, [buf[s:s + n].numpy() for s, n in zip(starts, sizes)]
+    host = buf.numpy()
+    return buf, [host[s:s + n] for s, n in zip(starts, sizes)]
 
 
-def _ends_equal(a, value):
-    return len(a) > 0 and a[0] == value and a[-1] == value
+# fractions spread evenly over [0, 1), without a period that an array could share
+_SPREAD = np.arange(1024) * ((5 ** .5 - 1) / 2) % 1
+
+
+def _unless(a, value):
+    """None for an int64 array whose every entry is ``value``, -1 or 0 (the rule), else
+    the array.  One pass (10 us for 65,536 rays, 45 for 262,144), left out where a
+    thousand entries (5 us) of a longer array show already that it is not."""
+    same = np.bitwise_and.reduce if value else np.bitwise_or.reduce
+    if not len(a) or len(a) > 65536 and same(a[(_SPREAD * len(a)).astype(np.int64)]) != value or same(a) != value:
+        return a
+    return None
+
+
+# Bytes of an int64 array up to which a copy in page-locked memory, read by the kernel over the link, costs less than
+# a copy to the device (65,536 rays: 17 us and 10 over the link against 53; 262,144: 133 and 38 against 154).
+_STAGE_BYTES = 1 << 20
+
+
+def _stage_bytes(a):
+    return 0 if a is None or a.nbytes > _STAGE_BYTES else a.nbytes
+
+
+def _staged(a, space, device, hold):
+    """Address of an int64 array that kernels can read: as _reachable, but a short
+    array is copied into ``space`` (page-locked, _stage_bytes)."""
+    if a is None:
+        return None
+    if not len(space) or torch().from_numpy(a).is_pinned():
+        return _reachable(a, device, hold)
+    space.view(np.int64)[...] = a
+    return space.ctypes.data
 
 
 class GPUEHSSTransport:
@@ -240,24 +272,14 @@ class GPUEHSSTransport:
             last, bounces = (_per_ray(a, np.int64, (n,)) for a in (source.last_atom, source.initial_bounces))
         except (ValueError, IndexError):
             raise ValueError('One origin, direction, initial identity and bounce count per weight required') from None
-        # A source starts without colliders (-1) and collisions as a rule.  Where its ends say so, the device traces
-        # it that way while the host reads the two arrays through; if an entry differs, the result is dropped and
-        # the arrays are checked and traced as they are.
-        done = None
-        if _ends_equal(last, -1) and _ends_equal(bounces, 0):
-            done = self._enqueue(origins, directions, None, None, cap, record_history)
-            plain = not bounces.any() and last.max() == -1 and last.min() == -1
-            torch().cuda.current_stream(self.scene.device).synchronize()
-            if not plain:
-                done = None
-        if done is None:
-            if np.any(source.initial_bounces > 1):
-                raise ValueError('Positive cap and zero/one initial collision required')
-            if np.any(last < -1) or np.any(last >= self.scene.n_atoms):
-                raise ValueError('Invalid initial physical identity')
-            done = self._enqueue(origins, directions, last, bounces, cap, record_history)
-            torch().cuda.current_stream(self.scene.device).synchronize()
-        (P, D, b, esc, unres, st), hist_out = done
+        # a source starts without colliders and collisions as a rule, and then needs neither array
+        last, bounces = _unless(last, -1), _unless(bounces, 0)
+        if bounces is not None and np.any(source.initial_bounces > 1):
+            raise ValueError('Positive cap and zero/one initial collision required')
+        if last is not None and (np.any(last < -1) or np.any(last >= self.scene.n_atoms)):
+            raise ValueError('Invalid initial physical identity')
+        (P, D, b, esc, unres, st), hist_out = self._enqueue(origins, directions, last, bounces, cap, record_history)
+        torch().cuda.current_stream(self.scene.device).synchronize()
         if st[_lib.STAT_ERRORS]:
             raise _lib.EHSSDeviceError(f'{int(st[_lib.STAT_ERRORS])} rays reported a bounded device failure')
         history = hist_out.numpy() if record_history else np.full((n, 0), -1, dtype=np.int32)
@@ -281,15 +303,17 @@ class GPUEHSSTransport:
         lib, t, dev = _lib.load(), torch(), self.scene.device
         n = len(origins)
         hold = []
-        inputs = [None if a is None else _reachable(a, dev, hold) for a in (origins, directions, last, bounces)]
+        rays = [_reachable(a, dev, hold) for a in (origins, directions)]
         wb = ct.c_uint64()
         _lib.check(lib.ehss_trace_host_workspace_bytes(n, ct.byref(wb)), 'trace')
         ws = t.empty(wb.value, dtype=t.uint8, device=dev)
-        buf, (P, D, b, esc, unres, st) = _page_locked(dev, (24 * n, 24 * n, 8 * n, n, n, 8 * _lib.NSTATS))
+        buf, (P, D, b, esc, unres, st, *space) = _page_locked(dev, (24 * n, 24 * n, 8 * n, n, n, 8 * _lib.NSTATS) + tuple(
+            map(_stage_bytes, (last, bounces))))
+        initial = [_staged(a, v, dev, hold) for a, v in zip((last, bounces), space)]
         hist = t.full((n, cap), -1, dtype=t.int32, device=dev) if record_history else None
         hist_out = t.empty((n, cap), dtype=t.int32, pin_memory=True) if record_history else None
         out = [a.ctypes.data for a in (P, D, b, esc, unres)]
-        _lib.check(lib.ehss_trace_host(self.scene.ptr, n, cap, self.precision, *inputs, *out, ptr(hist), st.ctypes.data,
+        _lib.check(lib.ehss_trace_host(self.scene.ptr, n, cap, self.precision, *rays, *initial, *out, ptr(hist), st.ctypes.data,
                                        ws.data_ptr(), wb.value, stream_handle(dev)), 'trace')
         if hist is not None:
             hist_out.copy_(hist, non_blocking=True)
@@ -366,18 +390,8 @@ class SphereIndex:
         n = len(source.origins)
         origins, directions = (_rows(a, np.float64, n, 3) for a in (source.origins, source.directions))
         own = _rows(owners, np.int64, n, 1).reshape(-1)
-        # rays without an owner (-1) are the rule: traced so while the host reads the owners through (as in trace)
-        done = None
-        if _ends_equal(own, -1):
-            done = self._enqueue(origins, directions, None)
-            plain = own.max() == -1 and own.min() == -1
-            torch().cuda.current_stream(self.scene.device).synchronize()
-            if not plain:
-                done = None
-        if done is None:
-            done = self._enqueue(origins, directions, own)
-            torch().cuda.current_stream(self.scene.device).synchronize()
-        blocked, st = done
+        blocked, st = self._enqueue(origins, directions, _unless(own, -1))
+        torch().cuda.current_stream(self.scene.device).synchronize()
         if st[_lib.STAT_ERRORS]:
             raise _lib.EHSSDeviceError('PA query reported a bounded device failure')
         return blocked, int(st[_lib.STAT_BOX]), int(st[_lib.STAT_SPHERE])
@@ -391,8 +405,9 @@ class SphereIndex:
         lib, t, dev = _lib.load(), torch(), self.scene.device
         n = len(origins)
         hold = []
-        P, D, own = (None if a is None else _reachable(a, dev, hold) for a in (origins, directions, owners))
-        buf, (blocked, st) = _page_locked(dev, (n, 8 * _lib.NSTATS))
+        P, D = (_reachable(a, dev, hold) for a in (origins, directions))
+        buf, (blocked, st, space) = _page_locked(dev, (n, 8 * _lib.NSTATS, _stage_bytes(owners)))
+        own = _staged(owners, space, dev, hold)
         stats = t.zeros(_lib.NSTATS, dtype=t.int64, device=dev)
         _lib.check(lib.ehss_pa_anyhit(self.scene.ptr, n, P, D, own, blocked.ctypes.data if n else None, ptr(stats),
                                       stream_handle(dev)), 'PA query')

@@ -64,4 +64,4 @@ def test_launch_on_the_scene_device(monkeypatch, call):
         index = engine.SphereIndex.__new__(engine.SphereIndex)
         index.scene = scene
         index.query(SimpleNamespace(origins=np.zeros((4, 3)), directions=d, owners=np.array([-1, 2, 2, -1])))
-    assert seen == ['cuda:1', 'cuda:1'] and fake.current() == 'cuda:0'
+    assert seen and set(seen) == {'cuda:1'} and fake.current() == 'cuda:0'
