@@ -390,7 +390,10 @@ class SphereIndex:
         n = len(source.origins)
         origins, directions = (_rows(a, np.float64, n, 3) for a in (source.origins, source.directions))
         own = _rows(owners, np.int64, n, 1).reshape(-1)
-        blocked, st = self._enqueue(origins, directions, _unless(own, -1))
+        # long rays that are copied to the device take their owners with them: the copy costs little more than the look
+        if n <= 65536 or torch().from_numpy(origins).is_pinned():
+            own = _unless(own, -1)
+        blocked, st = self._enqueue(origins, directions, own)
         torch().cuda.current_stream(self.scene.device).synchronize()
         if st[_lib.STAT_ERRORS]:
             raise _lib.EHSSDeviceError('PA query reported a bounded device failure')
