@@ -397,7 +397,8 @@ class SphereIndex:
         torch().cuda.current_stream(self.scene.device).synchronize()
         if st[_lib.STAT_ERRORS]:
             raise _lib.EHSSDeviceError('PA query reported a bounded device failure')
-        return blocked, int(st[_lib.STAT_BOX]), int(st[_lib.STAT_SPHERE])
+        # an array of its own: the page-locked buffer serves the next call, also while the caller keeps the result
+        return blocked.copy(), int(st[_lib.STAT_BOX]), int(st[_lib.STAT_SPHERE])
 
     def _enqueue(self, origins, directions, owners):
         """Enqueue one any-hit query (no wait); returns the host arrays that it fills."""
