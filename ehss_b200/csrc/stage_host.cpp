@@ -6,8 +6,12 @@
 // numpy's and the device builder's do.
 #include <atomic>
 #include <cmath>
+#include <cstdint>
 #include <cstring>
 #include <thread>
+#if defined(__x86_64__)
+#include <emmintrin.h>
+#endif
 #include "../../include/ehss_b200.h"
 
 namespace ehss {
@@ -30,6 +34,20 @@ void enclosing_sphere(int64_t n, const double* xyz, const double* radii, double*
         most = len > most ? len : most;
     }
     *radius = nan ? NAN : most * 1.000000001;
+}
+
+// Copy into a page-locked buffer, past the caches: lines that several cores hold modified slow the upload that reads
+// them next (40 structures of 5000 atoms staged by several threads: 130 us of upload became 170 to 300).
+static void copy_out(double* dst, const double* src, int64_t n) {
+#if defined(__x86_64__)
+    int64_t i = 0;
+    if (n > 0 && ((uintptr_t)dst & 15u)) { dst[0] = src[0]; i = 1; }
+    for (; i + 2 <= n; i += 2) _mm_stream_pd(dst + i, _mm_loadu_pd(src + i));
+    if (i < n) dst[i] = src[i];
+    _mm_sfence();
+#else
+    std::memcpy(dst, src, sizeof(double) * (size_t)n);
+#endif
 }
 
 // Runs f(0) .. f(count - 1), on up to `threads` threads; a thread that cannot be started is done without.
@@ -87,8 +105,8 @@ extern "C" int ehss_stage_structures(int n_structures, const double* const* xyz,
         int64_t at = 0;
         for (int s = 0; s < first; ++s) at += n_atoms[s];
         for (int s = first; s < end; ++s) {
-            std::memcpy(xyz_out + 3 * at, xyz[s], 24 * (size_t)n_atoms[s]);
-            std::memcpy(radii_out + at, radii[s], 8 * (size_t)n_atoms[s]);
+            copy_out(xyz_out + 3 * at, xyz[s], 3 * n_atoms[s]);
+            copy_out(radii_out + at, radii[s], n_atoms[s]);
             at += n_atoms[s];
         }
     });
