@@ -744,8 +744,8 @@ def main():
     if rank == 0:
         # builder: two passes around the exposure test, every structure here holding at most 8192 atoms;
         # more than 8 structures: scene index + stats, 5 tree kernels a pass (keys sorted per structure in
-        # one kernel), a fix-up behind the exposure test; up to 8: one tree kernel (one CTA a structure) and
-        # two emission kernels a pass.  Then 1 persistent trace kernel
+        # one kernel), a fix-up behind the exposure test; up to 8 (of at most 6144 atoms, as
+        # all here): one tree kernel (one CTA a structure) and two emission kernels a pass.  Then 1 persistent trace kernel
         launches_per_step = (2 + 5 * 2 + 2 if len(structures) > 8 else 3 * 2 + 1) + 1
         line = {"metric": METRIC, "value": value, "unit": UNIT, "n_gpus": world, "steps": args.steps,
                 "warmup": args.warmup, "ms_per_step": total_ms / args.steps, "higher_is_better": True,

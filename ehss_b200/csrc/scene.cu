@@ -30,7 +30,7 @@
 //                  by eps_box; subtrees of at most leaf_size atoms collapsed
 //                  into leaf references); per atom: FP32 and FP64 records in
 //                  leaf order, id maps.
-// Up to 8 structures of at most 8192 atoms: steps 1-5 in one launch, one CTA a
+// Up to 8 structures of at most 6144 atoms: steps 1-5 in one launch, one CTA a
 // structure (k_build_small).
 // Exterior builds (EHSS_BUILD_EXTERIOR) then run k_exposure on that tree and
 // repeat steps 2-6 with the buried atoms sorted behind the exposed ones and
@@ -686,7 +686,7 @@ __global__ void k_emit_atoms(const BuildDesc* descs, const int32_t* atom_scene, 
 }
 
 // --------------------------------------------------------------------------
-// Up to kOneCtaTrees structures, all of at most kSegSortMax atoms: one CTA makes
+// Up to kOneCtaTrees structures, all of at most kOneCtaAtoms atoms: one CTA makes
 // one structure's tree in one launch (a launch a pass: the full tree, and for
 // exterior scenes the tree over the exposed atoms after k_exposure), and
 // k_emit_nodes and k_emit_atoms write the records on all SMs.  The phases are those of the device-wide path
@@ -728,6 +728,9 @@ struct SmallBuild {
 // launches are what a build costs, by up to 1.7 times; in a batch by 4 to 9 % of a build that is a tenth of the step.
 // Batches keep the 15 launches a step that bench.py states and its test expects.
 constexpr int kOneCtaTrees = 8;
+// Most atoms of such a structure: from about 6500 on one CTA's sort and walk take longer than the launches that they
+// replace (one scene of 6000, 7000 and 8192 atoms, passes / one CTA: 293 / 292, 310 / 323, 332 / 357 us).
+constexpr int kOneCtaAtoms = 6144;
 constexpr int kNoParent = 0xffff;
 constexpr unsigned kNobody = 0xffffffffu, kIsLeaf = 0x80000000u;
 
@@ -1573,7 +1576,7 @@ int build_scenes(int S, const double* const* xyz, const double* const* radii, co
 
     const int T = 256;
     auto blocks = [&](int64_t count) { return (unsigned)((count + T - 1) / T); };
-    const bool segsort = max_n <= kSegSortMax, small = segsort && S <= kOneCtaTrees;
+    const bool segsort = max_n <= kSegSortMax, small = max_n <= kOneCtaAtoms && S <= kOneCtaTrees;
     if (!small) {
         k_fill_scene_index<<<S, 256, 0, stream>>>(W.descs, S, W.atom_scene);
         k_stats<<<S, 256, 0, stream>>>(W.descs, S);

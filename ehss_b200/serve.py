@@ -221,8 +221,8 @@ class DeviceExecutor:
     def warmup(self, sizes=(64, 4096, 12000)):
         """Build and trace one synthetic structure of each size, then build by
         the paths that those do not take (scene.cu: one CTA a structure in three
-        sizes, up to 1024, 2048 and 8192 atoms, for up to 8 structures; key sorts
-        a structure in two sizes for more; the device-wide sort above 8192 atoms),
+        sizes, up to 1024, 2048 and 6144 atoms, for up to 8 structures; key sorts
+        a structure in two sizes for others; the device-wide sort above 8192 atoms),
         so that the first requests do not wait for kernels to load."""
         rng = np.random.default_rng(0)
 

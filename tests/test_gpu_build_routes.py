@@ -1,5 +1,5 @@
-"""Batches on either side of the number of structures up to which one CTA makes
-each tree: a structure's scene is the same byte for byte in both."""
+"""Batches on either side of the numbers of structures and atoms up to which one
+CTA makes each tree: a structure's scene is the same byte for byte in both."""
 import numpy as np
 import pytest
 
@@ -12,7 +12,7 @@ def _bytes(batch, i):
 
 
 @pytest.mark.parametrize('exterior', [False, True])
-@pytest.mark.parametrize('largest', [3, 1024, 2048, 2049, 8192])
+@pytest.mark.parametrize('largest', [3, 1024, 2048, 2049, 6144, 6145, 8192])
 def test_eight_and_nine_structures(largest, exterior):
     from ehss_b200 import workloads as W
     from ehss_b200.batch import BatchScenes
