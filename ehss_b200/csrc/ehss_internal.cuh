@@ -54,8 +54,7 @@ struct alignas(256) SceneHeader {
     double rmax;
     float eps_box;         // absolute FP32 box expansion
     float scale_f;
-    float rmax_f;
-    float pad0;
+    float pad0, pad1;
     int32_t n_active;      // atoms in the tree: all of them, or the exposed ones of an exterior scene
     int32_t exterior;      // 1: buried atoms left out of the tree (valid for rays starting outside)
     uint64_t off_nodes, off_atoms, off_atoms64, off_ids, off_rank;

@@ -94,8 +94,8 @@ struct BuildWork {
 constexpr int kSumRows = 256;        // atoms of one chunk of the sequential coordinate sum
 
 // Header, centre, extents and input checks of one structure, by one CTA.
-// Returns false (to every thread) for a refit of a scene that cannot be refit.
-__device__ __forceinline__ bool scene_stats(BuildDesc& D) {
+// A refit of a scene that cannot be refit ends with the scene's status set.
+__device__ __forceinline__ void scene_stats(BuildDesc& D) {
     SceneHeader* H = reinterpret_cast<SceneHeader*>(D.scene);
     const int64_t n = D.n;
     __shared__ double center[3];
@@ -114,7 +114,7 @@ __device__ __forceinline__ bool scene_stats(BuildDesc& D) {
             bad = 0;
         }
         __syncthreads();
-        if (mismatch) return false;
+        if (mismatch) return;
     } else {
         // header: zeroed, then the layout offsets (the rest is filled below and by k_emit_nodes)
         if (threadIdx.x < sizeof(SceneHeader) / 4) reinterpret_cast<uint32_t*>(H)[threadIdx.x] = 0u;
@@ -222,7 +222,6 @@ __device__ __forceinline__ bool scene_stats(BuildDesc& D) {
         H->scale = result[1];
         H->radius = dmul(result[1], 1.000000001);
         H->scale_f = __double2float_ru(result[1]);
-        H->rmax_f = __double2float_ru(result[0]);
         // FP32 box expansion: 2^-14 S covers the FP32 rounding of any ray
         // whose origin lies within 3 S of the centre (the traversal sends
         // farther origins to the FP64 all-atom search).
@@ -233,7 +232,6 @@ __device__ __forceinline__ bool scene_stats(BuildDesc& D) {
         }
     }
     __syncthreads();
-    return true;
 }
 
 __global__ void k_stats(BuildDesc* descs, int n_scenes) {

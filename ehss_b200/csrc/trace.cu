@@ -846,8 +846,7 @@ __device__ __forceinline__ int resolve_candidates(const SceneView& S, const Walk
 // (one in 450,000 on the mixed 256-globule batch) or cannot be walked in FP32,
 // and the warp takes the parked rays when no lane is in a query: as a call in the
 // resolve phase, every value that a lane holds across it was stored and
-// reloaded on the hot path (88 / 116 B of spills a thread, 10 % of the batched
-// trace).  Inlined here, where no value of a query is live; as a call it still
+// reloaded on the hot path (10 % of the batched trace).  Inlined here, where no value of a query is live; as a call it still
 // cost 4 %.  Returns whether the ray escaped.
 template <bool UNIT>
 __device__ __forceinline__ bool rest_of_path(const void* scene, LaneRay& L, int cap, int& bounces, int& last_rank,
@@ -908,7 +907,7 @@ __device__ __forceinline__ bool next_chunk(unsigned long long* counters, int n_p
 // PA: the instance that serves EHSS_BLOCK_PA; the caller says with
 // EHSS_LAUNCH_NO_PA that no block has it (such a block is then an error), which
 // keeps the any-hit query's registers out of the kernel (spill stores / loads a
-// thread 112 / 164 -> 88 / 116 B; the 256-globule batch 2 % faster).
+// thread 174 / 230 -> 116 / 156 B; the 256-globule batch 2 % faster).
 template <bool EXACT, bool COUNT, bool RAYS, bool PA>
 __global__ void __launch_bounds__(128, 8) k_blocks(const ehss_block* blocks, int nb, int64_t chunk_first,
                                                    int64_t total_chunks, int chunk_rays, int resolve_batch,

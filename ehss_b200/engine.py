@@ -145,8 +145,7 @@ def external_source(spheres, power, seed, scene=None):
 
     Same contract as the reference's external_source: 2**power rays, weight
     pi R^2 / n each, no initial collider.  The ray arrays are numpy arrays
-    over page-locked host memory, so handing them back to a trace copies them
-    to the device by DMA.
+    over page-locked host memory, which a trace reads where they lie.
     """
     power = int(power)
     if not 0 <= power <= 30:
@@ -155,7 +154,7 @@ def external_source(spheres, power, seed, scene=None):
     scene = scene or Scene.from_spheres(spheres)
     o, d = scene.source_rays(power, seed)
     t = torch()
-    # page-locked host arrays: the copy back and a later trace's copy in run as DMA
+    # page-locked host arrays: the copy back runs as DMA, and a later trace reads them in place
     host = t.empty((3, o.shape[0], 3), dtype=t.float64, pin_memory=True)
     host[0].copy_(o, non_blocking=True)
     host[1].copy_(d, non_blocking=True)

@@ -150,7 +150,8 @@ int ehss_scenes_build_ex(int n_scenes, const double* const* xyz_dev, const doubl
 /* ehss_scenes_build_ex with the structures' centres given: centers_host[3 n]
  * holds each one's mean, summed in row order as ehss_stage_structures does (the
  * device's own chain of that many dependent additions is most of a small
- * build's statistics).  Everything else is computed from the coordinates. */
+ * build's statistics).  Everything else is computed from the coordinates,
+ * whose centres these must be. */
 int ehss_scenes_build_centred(int n_scenes, const double* const* xyz_dev, const double* const* radii_dev,
                               const int64_t* n_atoms_host, int leaf_size, void* const* scenes_dev,
                               const uint64_t* scene_bytes_host, void* workspace_dev, uint64_t workspace_bytes,
@@ -243,7 +244,7 @@ int ehss_trace(const void* scene_dev, int64_t n_rays, int cap, int precision,
  * host while others are traced.  origins/directions [n*3], last_atom and
  * initial_bounces [n] (NULL: -1 and 0 for every ray) and the result arrays
  * must lie in page-locked host memory (cudaHostAlloc, cudaHostRegister) or
- * device memory; anything else is EHSS_ERR_VALUE.  The source arrays are not
+ * device memory, aligned as their elements; anything else is EHSS_ERR_VALUE.  The source arrays are not
  * written.  history_dev as in ehss_trace.  stats_host (page-locked
  * uint64[EHSS_NSTATS]) receives this call's counters.  Results are complete
  * when `stream` is.  workspace_dev holds at least
@@ -259,7 +260,9 @@ int ehss_trace_host(const void* scene_dev, int64_t n_rays, int cap, int precisio
  * (pa_spatial.py:133-142, 162-164) with sphere_hit semantics
  * (inside_out_pa.py:93-101): blocked_dev[i] = 1 when ray i meets a sphere
  * other than owners_dev[i] (NULL = no owner).  The arrays may also lie in
- * page-locked host memory. */
+ * page-locked host memory; their addresses must be aligned as their elements
+ * (EHSS_ERR_VALUE otherwise).  sphere_hit takes |d| = 1; for directions of
+ * another length the result is what its formula gives over every atom. */
 int ehss_pa_anyhit(const void* scene_dev, int64_t n_rays, const double* origins_dev, const double* directions_dev,
                    const int64_t* owners_dev, uint8_t* blocked_dev, uint64_t* stats_dev, void* stream);
 
