@@ -211,23 +211,44 @@ def _page_locked(device, sizes):
     return buf, [host[s:s + n] for s, n in zip(starts, sizes)]
 
 
+# Rays from which on a pass over an array of them (65,536: 8 us where they are in a cache, 37 where not; 262,144: 36 and
+# 132) is made while the device works.
+_LONG = 65536
 # fractions spread evenly over [0, 1), without a period that an array could share
 _SPREAD = np.arange(1024) * ((5 ** .5 - 1) / 2) % 1
 
 
+def _all(a, value):
+    """Whether every entry of an int64 array is ``value``, -1 or 0."""
+    return len(a) > 0 and (np.bitwise_and if value else np.bitwise_or).reduce(a) == value
+
+
+def _seems_all(a, value):
+    """The same of a thousand entries (5 us)."""
+    return _all(a[(_SPREAD * len(a)).astype(np.int64)], value)
+
+
 def _unless(a, value):
-    """None for an int64 array whose every entry is ``value``, -1 or 0 (the rule), else
-    the array.  One pass (10 us for 65,536 rays, 45 for 262,144), left out where a
-    thousand entries (5 us) of a longer array show already that it is not."""
-    same = np.bitwise_and.reduce if value else np.bitwise_or.reduce
-    if not len(a) or len(a) > 65536 and same(a[(_SPREAD * len(a)).astype(np.int64)]) != value or same(a) != value:
-        return a
-    return None
+    """None for an int64 array whose every entry is ``value``, -1 or 0 (the rule), else the
+    array.  One pass, left out where a sample of a long array shows that it is not."""
+    return None if (len(a) <= _LONG or _seems_all(a, value)) and _all(a, value) else a
 
 
 # Bytes of an int64 array up to which a copy in page-locked memory, read by the kernel over the link, costs less than
 # a copy to the device (65,536 rays: 17 us and 10 over the link against 53; 262,144: 133 and 38 against 154).
 _STAGE_BYTES = 1 << 20
+
+
+def _ahead(a, device, hold):
+    """Address of a device copy of a long page-locked array, which crosses the link
+    while the host reads others through (_unless; 262,144 traced rays of 2000 atoms:
+    911 us, read where they lie after that 1000); None for any other array."""
+    host = torch().from_numpy(a)
+    if len(a) <= _LONG or not host.is_pinned():
+        return None
+    with torch().cuda.device(device):
+        hold.append(host.to(device, non_blocking=True))
+    return hold[-1].data_ptr()
 
 
 def _stage_bytes(a):
@@ -250,8 +271,9 @@ class GPUEHSSTransport:
 
     ``trace`` takes and returns host arrays, as the reference does.  One
     launch reads the rays from page-locked host memory (rays in pageable
-    arrays are copied to the device first), traces them and writes the results
-    into a page-locked buffer whose parts become the returned arrays.
+    arrays, and more than 65,536 of them, are copied to the device first),
+    traces them and writes the results into a page-locked buffer whose parts
+    become the returned arrays.
     """
 
     def __init__(self, scene, precision='fp32', threads=1):
@@ -271,14 +293,19 @@ class GPUEHSSTransport:
             last, bounces = (_per_ray(a, np.int64, (n,)) for a in (source.last_atom, source.initial_bounces))
         except (ValueError, IndexError):
             raise ValueError('One origin, direction, initial identity and bounce count per weight required') from None
-        # a source starts without colliders and collisions as a rule, and then needs neither array
-        last, bounces = _unless(last, -1), _unless(bounces, 0)
-        if bounces is not None and np.any(source.initial_bounces > 1):
-            raise ValueError('Positive cap and zero/one initial collision required')
-        if last is not None and (np.any(last < -1) or np.any(last >= self.scene.n_atoms)):
-            raise ValueError('Invalid initial physical identity')
-        (P, D, b, esc, unres, st), hist_out = self._enqueue(origins, directions, last, bounces, cap, record_history)
-        torch().cuda.current_stream(self.scene.device).synchronize()
+        wait = torch().cuda.current_stream(self.scene.device).synchronize
+        hold = []
+        try:
+            ahead = [_ahead(a, self.scene.device, hold) for a in (origins, directions)]
+            # a source starts without colliders and collisions as a rule, and then needs neither array
+            last, bounces = _unless(last, -1), _unless(bounces, 0)
+            if bounces is not None and np.any(source.initial_bounces > 1):
+                raise ValueError('Positive cap and zero/one initial collision required')
+            if last is not None and (np.any(last < -1) or np.any(last >= self.scene.n_atoms)):
+                raise ValueError('Invalid initial physical identity')
+            (P, D, b, esc, unres, st), hist_out = self._enqueue(ahead, origins, directions, last, bounces, cap, record_history)
+        finally:
+            wait()
         if st[_lib.STAT_ERRORS]:
             raise _lib.EHSSDeviceError(f'{int(st[_lib.STAT_ERRORS])} rays reported a bounded device failure')
         history = hist_out.numpy() if record_history else np.full((n, 0), -1, dtype=np.int32)
@@ -292,17 +319,17 @@ class GPUEHSSTransport:
                                threads=self.threads, history_recorded=bool(record_history),
                                response_reuse=False))
 
-    def _enqueue(self, origins, directions, last, bounces, cap, record_history):
+    def _enqueue(self, ahead, origins, directions, last, bounces, cap, record_history):
         """Enqueue one trace (no wait); returns the host arrays that it fills."""
         # the scene's device, whichever is the thread's current one: the handle of a default stream names no device
         with torch().cuda.device(self.scene.device):
-            return self._launch(origins, directions, last, bounces, cap, record_history)
+            return self._launch(ahead, origins, directions, last, bounces, cap, record_history)
 
-    def _launch(self, origins, directions, last, bounces, cap, record_history):
+    def _launch(self, ahead, origins, directions, last, bounces, cap, record_history):
         lib, t, dev = _lib.load(), torch(), self.scene.device
         n = len(origins)
         hold = []
-        rays = [_reachable(a, dev, hold) for a in (origins, directions)]
+        rays = [p or _reachable(a, dev, hold) for p, a in zip(ahead, (origins, directions))]
         wb = ct.c_uint64()
         _lib.check(lib.ehss_trace_host_workspace_bytes(n, ct.byref(wb)), 'trace')
         ws = t.empty(wb.value, dtype=t.uint8, device=dev)
@@ -389,9 +416,6 @@ class SphereIndex:
         n = len(source.origins)
         origins, directions = (_rows(a, np.float64, n, 3) for a in (source.origins, source.directions))
         own = _rows(owners, np.int64, n, 1).reshape(-1)
-        # long rays that are copied to the device take their owners with them: the copy costs little more than the look
-        if n <= 65536 or torch().from_numpy(origins).is_pinned():
-            own = _unless(own, -1)
         blocked, st = self._enqueue(origins, directions, own)
         torch().cuda.current_stream(self.scene.device).synchronize()
         if st[_lib.STAT_ERRORS]:
@@ -408,7 +432,13 @@ class SphereIndex:
         lib, t, dev = _lib.load(), torch(), self.scene.device
         n = len(origins)
         hold = []
-        P, D = (_reachable(a, dev, hold) for a in (origins, directions))
+        # Rays without owners are the rule (_unless); rays that are copied to the device take theirs with them from where
+        # that copy costs little more than the look.  The origins are enough to cross the link ahead: the look takes less
+        # than those of a trace (200,000 rays: 313 us, with nothing ahead 400).
+        P = _ahead(origins, dev, hold)
+        if P or n <= 16384 or t.from_numpy(origins).is_pinned():
+            owners = _unless(owners, -1)
+        P, D = P or _reachable(origins, dev, hold), _reachable(directions, dev, hold)
         buf, (blocked, st, space) = _page_locked(dev, (n, 8 * _lib.NSTATS, _stage_bytes(owners)))
         own = _staged(owners, space, dev, hold)
         stats = t.zeros(_lib.NSTATS, dtype=t.int64, device=dev)

@@ -38,7 +38,8 @@ class _Torch:
 
     def from_numpy(self, a):
         t = real.from_numpy(a)
-        return SimpleNamespace(is_pinned=lambda: True, data_ptr=t.data_ptr, copy_=lambda other, **kw: t.copy_(other))
+        return SimpleNamespace(is_pinned=lambda: True, data_ptr=t.data_ptr, copy_=lambda other, **kw: t.copy_(other),
+                               to=lambda device, **kw: t)
 
     def __getattr__(self, name):
         return getattr(real, name)

@@ -11,7 +11,8 @@ from ehss_b200 import _lib, engine
 
 
 @pytest.mark.parametrize('call', ['trace', 'query'])
-@pytest.mark.parametrize('n,differ', [(1, 0), (3000, 0), (3000, 1000), (3000, 1), (40000, 0), (40000, 13000), (40000, 2)])
+@pytest.mark.parametrize('n,differ', [(1, 0), (3000, 0), (3000, 1000), (3000, 1), (40000, 0), (40000, 13000), (40000, 2), (70000, 0),
+                                      (70000, 23000), (70000, 2)])
 def test_rays_are_launched_once(monkeypatch, call, n, differ):
     fake, launched = _Torch(), []
     lib = SimpleNamespace(
@@ -45,3 +46,7 @@ def test_uniform_arrays(value):
             a[n // 2] = other
             assert engine._unless(a, value) is a
     assert engine._unless(np.empty(0, dtype=np.int64), value) is not None
+    a = np.full(100000, value)
+    assert engine._unless(a, value) is None and engine._seems_all(a, value)
+    a[::3] = 7
+    assert engine._unless(a, value) is a and not engine._seems_all(a, value)
